@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(DS_THREADS) k_dd_sums(FmDev d, double *out)
     for (int k = 0; k < RS_N; k++) { sum[k] = 0.0; cmp[k] = 0.0; }
     for (int b = threadIdx.x; b < d.nblocks_force; b += DS_THREADS) {
         for (int k = 0; k < RS_N; k++) {
+            if (k >= RS_PXX && !d.pressure) break;  // not summed, not written
             const double v = d.partial[(size_t)b * RS_N + k];
             if (k == RS_PEMAX) { sum[k] = fmax(sum[k], v); continue; }
             neumaier(sum[k], cmp[k], v);

@@ -1014,8 +1014,10 @@ __device__ __forceinline__ void block_partials(const FmDev &d, double v[RS_N], i
 {
     __shared__ double ws[RS_N][NT / 32], wc[RS_N][NT / 32];
     int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int nq = d.pressure ? (int)RS_N : (int)RS_PXX;  // the pressure terms only where they are summed
 #pragma unroll
     for (int k = 0; k < RS_N; k++) {
+        if (k >= nq) break;
         double x = v[k], c = 0.0;
         if (k == RS_PEMAX) {
             x = warp_max(x);
@@ -1029,7 +1031,7 @@ __device__ __forceinline__ void block_partials(const FmDev &d, double v[RS_N], i
         if (l == 0) { ws[k][w] = x; wc[k][w] = c; }
     }
     __syncthreads();
-    if (threadIdx.x < RS_N) {
+    if (threadIdx.x < nq) {
         int k = threadIdx.x;
         double acc = ws[k][0], cmp = wc[k][0];
         for (int q = 1; q < NT / 32; q++) {
@@ -1422,43 +1424,56 @@ __global__ void k_tile_to_generic(FmDev d, int32_t *out, int maxn)
 
 // Neumaier-compensated reduction of the per-block partials into one record
 // (evaluate_macroscopic_properties, simulation_record.f90:1205-1314).
-constexpr int REC_THREADS = 256;
+// One block: every thread sums a share of the rows, the warps merge by a fixed
+// xor tree and one thread per quantity merges the warps, so that nothing
+// longer than a few dozen merges is ever waited for (one thread merging all
+// 256 took 47-72 us a record step, whatever the system's size).
+constexpr int REC_THREADS = 512;
 __global__ void __launch_bounds__(REC_THREADS) k_record(FmDev d, int iter, double simtime)
 {
     pdl_enter();
     if (frozen(d)) return;
-    __shared__ double ssum[RS_N][REC_THREADS], scmp[RS_N][REC_THREADS];
+    __shared__ double ws[RS_N][REC_THREADS / 32], wc[RS_N][REC_THREADS / 32], tot[RS_N];
+    const int nq = d.pressure ? (int)RS_N : (int)RS_PXX;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double sum[RS_N], cmp[RS_N];
+#pragma unroll
     for (int k = 0; k < RS_N; k++) { sum[k] = 0.0; cmp[k] = 0.0; }
     for (int b = threadIdx.x; b < d.nblocks_force; b += REC_THREADS) {
+#pragma unroll
         for (int k = 0; k < RS_N; k++) {
-            double x = d.partial[(size_t)b * RS_N + k];
-            if (k == RS_PEMAX) { sum[k] = fmax(sum[k], x); continue; }
-            double t = sum[k] + x;
-            cmp[k] += fabs(sum[k]) >= fabs(x) ? (sum[k] - t) + x : (x - t) + sum[k];
-            sum[k] = t;
+            if (k >= nq) break;
+            const double x = d.partial[(size_t)b * RS_N + k];
+            if (k == RS_PEMAX) sum[k] = fmax(sum[k], x);
+            else neumaier(sum[k], cmp[k], x);
         }
     }
-    for (int k = 0; k < RS_N; k++) { ssum[k][threadIdx.x] = sum[k]; scmp[k][threadIdx.x] = cmp[k]; }
+#pragma unroll
+    for (int k = 0; k < RS_N; k++) {
+        if (k >= nq) break;
+        if (k == RS_PEMAX) {
+            sum[k] = warp_max(sum[k]);
+        } else {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const double s2 = __shfl_xor_sync(0xffffffffu, sum[k], o), c2 = __shfl_xor_sync(0xffffffffu, cmp[k], o);
+                nmerge(sum[k], cmp[k], s2, c2);
+            }
+        }
+        if (lane == 0) { ws[k][w] = sum[k]; wc[k][w] = cmp[k]; }
+    }
+    __syncthreads();
+    if (threadIdx.x < nq) {
+        const int k = threadIdx.x;
+        double s = ws[k][0], c = wc[k][0];
+        for (int q = 1; q < REC_THREADS / 32; q++) {
+            if (k == RS_PEMAX) s = fmax(s, ws[k][q]);
+            else nmerge(s, c, ws[k][q], wc[k][q]);
+        }
+        tot[k] = s + c;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        double tot[RS_N];
-        for (int k = 0; k < RS_N; k++) {
-            double s = 0.0, c = 0.0;
-            if (k == RS_PEMAX) {
-                for (int q = 0; q < REC_THREADS; q++) s = fmax(s, ssum[k][q]);
-                tot[k] = s;
-                continue;
-            }
-            for (int q = 0; q < REC_THREADS; q++) {
-                double x = ssum[k][q];
-                double t = s + x;
-                c += fabs(s) >= fabs(x) ? (s - t) + x : (x - t) + s;
-                s = t;
-                c += scmp[k][q];
-            }
-            tot[k] = s + c;
-        }
         const double gnp = (double)d.n;
         FmRecord r;
         r.iter = iter;
@@ -1522,13 +1537,13 @@ __global__ void __launch_bounds__(MACRO_THREADS) k_macro_partials(FmDev d)
 
 constexpr int AP_THREADS = 128;
 template <bool REC, int MODE, int PREC>
-__global__ void __launch_bounds__(AP_THREADS) k_all_pairs(FmDev d)
+__global__ void __launch_bounds__(AP_THREADS) k_all_pairs(FmDev d, int lanes)
 {
     pdl_enter();
     if (frozen(d)) return;
     const int pset = d.sc->pset;
     const double4 *P = cur_pos(d, pset);
-    const int i = blockIdx.x * AP_THREADS + threadIdx.x;
+    const int i = (blockIdx.x * AP_THREADS + threadIdx.x) / lanes, lane = threadIdx.x % lanes;
     const bool active = i < d.n;
     __shared__ double4 tile[AP_THREADS];
     double4 pi = active ? P[i] : make_double4(0, 0, 0, 0);
@@ -1539,7 +1554,7 @@ __global__ void __launch_bounds__(AP_THREADS) k_all_pairs(FmDev d)
         __syncthreads();
         int m = min(AP_THREADS, d.n - t0);
         if (active) {
-            for (int q = 0; q < m; q++) {
+            for (int q = lane; q < m; q += lanes) {
                 if (t0 + q == i) continue;
                 double4 pj = tile[q];
                 double r[3] = {__dsub_rn(pi.x, pj.x), __dsub_rn(pi.y, pj.y), __dsub_rn(pi.z, pj.z)};
@@ -1554,10 +1569,19 @@ __global__ void __launch_bounds__(AP_THREADS) k_all_pairs(FmDev d)
         }
         __syncthreads();
     }
+    for (int o = lanes >> 1; o > 0; o >>= 1) {
+        fx += __shfl_xor_sync(0xffffffffu, fx, o);
+        fy += __shfl_xor_sync(0xffffffffu, fy, o);
+        fz += __shfl_xor_sync(0xffffffffu, fz, o);
+        if (REC) {
+            pe += __shfl_xor_sync(0xffffffffu, pe, o);
+            vir += __shfl_xor_sync(0xffffffffu, vir, o);
+        }
+    }
     double part[RS_N] = {};
     double m2 = 0.0;
     const double rf[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // simulation_compute_forces_LJ_AP records no rf
-    if (active) m2 = epilogue<REC, MODE, (PREC & 2) != 0>(d, pset, i, pi, fx, fy, fz, pe, vir, part, rf);
+    if (active && lane == 0) m2 = epilogue<REC, MODE, (PREC & 2) != 0>(d, pset, i, pi, fx, fy, fz, pe, vir, part, rf);
     if (REC) block_partials<AP_THREADS>(d, part, blockIdx.x);
     if (MODE >= 2) block_vmax2(d, m2);
 }
@@ -1830,7 +1854,10 @@ void launch_tile_to_generic(const FmDev &d, int32_t *out, int maxn, cudaStream_t
 }
 
 int force_blocks(int n, int tpm) { return nblk(n * tpm, FORCE_THREADS); }
-int all_pairs_blocks(int n) { return nblk(n, AP_THREADS); }
+// Lanes per molecule: one lane's walk over all the others is what a small
+// system waits for (500 molecules: 85 us a step with one lane on two SMs).
+static int all_pairs_lanes(int n) { return n <= 8192 ? 32 : n <= 32768 ? 8 : 1; }
+int all_pairs_blocks(int n) { return nblk((long long)n * all_pairs_lanes(n), AP_THREADS); }
 
 template <int TPM>
 static void launch_force_tpm(const FmDev &d, int record, int mode, cudaStream_t st)
@@ -1873,14 +1900,14 @@ void launch_force(const FmDev &d, int record, int mode, int tpm, cudaStream_t st
 
 void launch_all_pairs(const FmDev &d, int record, int mode, cudaStream_t st)
 {
-    const int g = all_pairs_blocks(d.n);
+    const int g = all_pairs_blocks(d.n), lanes = all_pairs_lanes(d.n);
 #define FM_AP_CASE(R, M)                                                            \
     if (record == R && mode == M) {                                                 \
         switch (d.precision + 2 * d.mie) {                                          \
-        case 0: pdl_launch(k_all_pairs<R, M, 0>, g, AP_THREADS, st, d); break;           \
-        case 1: pdl_launch(k_all_pairs<R, M, 1>, g, AP_THREADS, st, d); break;           \
-        case 2: pdl_launch(k_all_pairs<R, M, 2>, g, AP_THREADS, st, d); break;           \
-        default: pdl_launch(k_all_pairs<R, M, 3>, g, AP_THREADS, st, d); break;          \
+        case 0: pdl_launch(k_all_pairs<R, M, 0>, g, AP_THREADS, st, d, lanes); break;           \
+        case 1: pdl_launch(k_all_pairs<R, M, 1>, g, AP_THREADS, st, d, lanes); break;           \
+        case 2: pdl_launch(k_all_pairs<R, M, 2>, g, AP_THREADS, st, d, lanes); break;           \
+        default: pdl_launch(k_all_pairs<R, M, 3>, g, AP_THREADS, st, d, lanes); break;          \
         }                                                                           \
         return;                                                                     \
     }
