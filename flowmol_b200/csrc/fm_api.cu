@@ -282,6 +282,7 @@ static int leave_tiles(fm_handle *h)
     if (d.nbr16) cudaFree(d.nbr16);
     d.nbr16 = nullptr;
     d.tile = 0;
+    d.build_rows = h->p.list_build == FM_LIST_BUILD_AUTO && h->cap <= fm::ROWS_MAX_MOLECULES ? 1 : 0;
     FM_TRY(alloc_nlist(h, maxn));
     return FM_OK;
 }
@@ -409,6 +410,7 @@ static int create_impl(const fm_params *p, const DdGeom *g, fm_handle **out)
     const double per_cell = rho * d.cs[0] * d.cs[1] * d.cs[2];
     d.build_blocks = p->list_build == FM_LIST_BUILD_BLOCKS ? 1
                      : p->list_build == FM_LIST_BUILD_CELLS ? 0 : (per_cell < 8.0 ? 1 : 0);
+    d.build_rows = p->list_build == FM_LIST_BUILD_AUTO && h->cap <= fm::ROWS_MAX_MOLECULES ? 1 : 0;
     int tpm = pick_tpm(*p, expected);
     if (g && p->threads_per_molecule == 0) h->p.threads_per_molecule = tpm;  // every rank the same kernel
     if (tpm < 0) { delete h; return fail(FM_ERR_ARG, "threads_per_molecule must be 0, 1, 2, 4, 8 or 16"); }
@@ -437,6 +439,7 @@ static int create_impl(const fm_params *p, const DdGeom *g, fm_handle **out)
         }
         if (want) {
             d.tile = 1;
+            d.build_rows = 0;  // staging offsets are the warp build's
             d.tile_T = p->threads_per_molecule == 4 ? 4 : p->threads_per_molecule == 8 ? 8 : (expected > 24 ? 8 : 4);
             d.tile_R = 3;  // (4 once Mie types or Soddemann bead flags are set; fixed at fm_setup)
             for (int k = 0; k < 3; k++) d.tile_nb[k] = (d.ne[k] + 1) / 2;

@@ -29,6 +29,13 @@
 // candidate order (all but its own entry, at distance 0), so every row lists
 // its partners in the visiting order.
 //
+// Bound by issue (81% of the slots at 1M molecules).  Pruned candidates are
+// collected across segments until 64 are there, so that no test or append
+// runs on a part-filled group but the last, and the owner lanes append two
+// groups' hits in one loop that writes sectors every eight steps: 738M -> 635M
+// instructions and 848 -> 709 us per 1M build (256 unpruned candidates a window,
+// one group and a sector check per append step before).
+//
 // With FENE polymers (POLY) the same scan discovers bonds the way the
 // reference's check_update_adjacentbeadinfo does (linklist.f90:2542-2584): any
 // candidate of the scanned cells -- at any distance -- with the owner's chain
@@ -50,10 +57,10 @@ namespace fm {
 
 constexpr int NB_WARPS = 4;                 // cells processed concurrently per block
 constexpr int NB_THREADS = 32 * NB_WARPS;
-constexpr int NB_STAGE = 256;               // staged candidates per warp
+constexpr int NB_STAGE = 96;                // staged candidates per warp: two halves of 32 and a step more
 constexpr int NB_OG = 4;                    // owners per step of the candidate loop
 constexpr int NB_CHUNK = 2;                 // work units a warp takes per fetch (one system)
-constexpr int NB_NOSHIFT = 1 | (1 << 2) | (1 << 4);
+constexpr int NB_RING = 16;                 // entries an owner lane buffers (power of two, two sectors)
 
 // One periodic system as the build sees it.  Molecule indices in entries,
 // rows and the per-molecule arrays count from the system's first molecule;
@@ -98,11 +105,11 @@ struct BuildShared {
     int start[54], code[54];
     int lbase[TILE ? 54 : 1];                   // segment k's first candidate in the block staging
     unsigned short loc[TILE ? NB_STAGE : 1];    // staged candidates' staging offsets
-    alignas(16) int ob[TILE ? 1 : 32][8];       // owner lane's chunk being filled (generic rows)
+    int ring[TILE ? 1 : NB_RING][32];           // entries an owner lane has not written yet (generic rows)
     alignas(16) unsigned short ob16[TILE ? 32 : 1][32];  // (tiled rows, 4 T <= 32 entries)
     int ochain[POLY ? 32 : 1];
     alignas(16) int4 obf[POLY ? 32 : 1];
-    unsigned hits[POLY ? 1 : 32];  // per owner: which of the 32 candidates hit (polymers: registers)
+    unsigned hits[POLY ? 1 : 2][32];  // per owner: which of the 32 candidates hit (polymers: registers)
 };
 
 constexpr uint32_t BUILD_OVER_LIST = 1u, BUILD_OVER_BONDS = 2u;
@@ -151,56 +158,82 @@ __device__ __forceinline__ bool exact_pair(const double4 *P, int io, int e, cons
     return norm2_rn(__dsub_rn(po.x, xj), __dsub_rn(po.y, yj), __dsub_rn(po.z, zj)) < rn2;
 }
 
-// Appends entry cnt (< maxn) of the owner (slot i) of this lane: into the
-// lane's chunk buffer, and the chunk to the row once it is full, so that every
-// sector of the row is written whole.  Generic rows: a chunk is 8 entries
-// (32 bytes) at nb_col(8c).  Tiled rows: a chunk is the 4 T entries of one load
-// of the owner's T lanes, contiguous at tile_pos16(4Tc), entry k at place
-// (k % T) 4 + (k / T) % 4 of it.
-template <bool TILE, typename SH>
-__device__ __forceinline__ void append_entry(SH &sh, int lane, int T, int32_t *nbr, uint16_t *row16, int i,
-                                             int maxn, int cnt, int ent, unsigned short loc)
+// Tiled rows: appends entry cnt (< maxn) of the owner of this lane into the
+// lane's chunk buffer, and the chunk to the row once it is full. A chunk is
+// the 4 T entries of one load of the owner's T lanes, contiguous at
+// tile_pos16(4Tc), entry k at place (k % T) 4 + (k / T) % 4 of it.
+template <typename SH>
+__device__ __forceinline__ void append_tile(SH &sh, int lane, int T, uint16_t *row16, int cnt, unsigned short loc)
 {
-    if (TILE) {
-        const int ch = 4 * T, k = cnt % ch;
-        sh.ob16[lane][(k % T) * 4 + (k / T) % 4] = loc;
-        if (k == ch - 1) {
-            const uint4 *src = reinterpret_cast<const uint4 *>(sh.ob16[lane]);
-            uint4 *dst = reinterpret_cast<uint4 *>(row16 + (cnt - k));
-            for (int q = 0; q < ch / 8; q++) dst[q] = src[q];
-        }
-    } else {
-        sh.ob[lane][cnt & 7] = ent;
-        if ((cnt & 7) == 7) {
-            const int4 *src = reinterpret_cast<const int4 *>(sh.ob[lane]);
-            int4 *dst = reinterpret_cast<int4 *>(nbr + nb_row(i, maxn) + nb_col(cnt & ~7));
-            dst[0] = src[0];
-            dst[1] = src[1];
-        }
+    const int ch = 4 * T, k = cnt % ch;
+    sh.ob16[lane][(k % T) * 4 + (k / T) % 4] = loc;
+    if (k == ch - 1) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(sh.ob16[lane]);
+        uint4 *dst = reinterpret_cast<uint4 *>(row16 + (cnt - k));
+        for (int q = 0; q < ch / 8; q++) dst[q] = src[q];
     }
 }
 
 // Writes the owner's last, partial chunk (cnt entries in all, cnt < maxn; the
-// chunk lies inside the row because maxn is a whole number of chunks).  Tiled
-// rows are padded with the dummy candidate up to the chunk's end, the force
-// kernel's last load; generic rows leave the places past cnt unread.
-template <bool TILE, typename SH>
-__device__ __forceinline__ void flush_entries(SH &sh, int lane, int T, int32_t *nbr, uint16_t *row16, int i,
-                                              int maxn, int cnt, int dummy)
+// chunk lies inside the row because maxn is a whole number of chunks), padded
+// with the dummy candidate up to its end, the force kernel's last load.
+template <typename SH>
+__device__ __forceinline__ void flush_tile(SH &sh, int lane, int T, uint16_t *row16, int cnt, int dummy)
 {
-    if (TILE) {
-        const int ch = 4 * T, k0 = cnt % ch;
-        if (k0 == 0) return;
-        for (int k = k0; k < ch; k++) sh.ob16[lane][(k % T) * 4 + (k / T) % 4] = (unsigned short)dummy;
-        const uint4 *src = reinterpret_cast<const uint4 *>(sh.ob16[lane]);
-        uint4 *dst = reinterpret_cast<uint4 *>(row16 + (cnt - k0));
-        for (int q = 0; q < ch / 8; q++) dst[q] = src[q];
-    } else {
-        if ((cnt & 7) == 0) return;
-        const int4 *src = reinterpret_cast<const int4 *>(sh.ob[lane]);
-        int4 *dst = reinterpret_cast<int4 *>(nbr + nb_row(i, maxn) + nb_col(cnt & ~7));
-        dst[0] = src[0];
-        dst[1] = src[1];
+    const int ch = 4 * T, k0 = cnt % ch;
+    if (k0 == 0) return;
+    for (int k = k0; k < ch; k++) sh.ob16[lane][(k % T) * 4 + (k / T) % 4] = (unsigned short)dummy;
+    const uint4 *src = reinterpret_cast<const uint4 *>(sh.ob16[lane]);
+    uint4 *dst = reinterpret_cast<uint4 *>(row16 + (cnt - k0));
+    for (int q = 0; q < ch / 8; q++) dst[q] = src[q];
+}
+
+// Generic rows: writes the sector (8 entries, 32 bytes, nb_col's order) of the
+// row that starts at entry `out` from the lane's ring; entries past the
+// row's last are left unread.
+template <typename SH>
+__device__ __forceinline__ void write_sector(SH &sh, int lane, int32_t *row, int out)
+{
+    int v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = sh.ring[(out & (NB_RING - 8)) + k][lane];
+    int4 *dst = reinterpret_cast<int4 *>(row + (size_t)out * 32u);
+    dst[0] = make_int4(v[0], v[4], v[1], v[5]);
+    dst[1] = make_int4(v[2], v[6], v[3], v[7]);
+}
+
+// The owner lanes append their hits among the staged candidates 0 .. 63 (bits
+// of m0, m1), in candidate order and without themselves, one each per step.
+// Two masks a time even out the lanes' counts (the loop runs as
+// long as the owner with the most hits), and sectors are written every eight
+// steps for all lanes that have one: with the full test and the write inside
+// the step some lane takes them nearly every time.
+template <typename SH>
+__device__ __forceinline__ void append_hits(SH &sh, int lane, unsigned m0, unsigned m1, int self_e, int32_t *row,
+                                            int maxn, int &cnt, int &out)
+{
+    int base = 0;
+    while (__any_sync(0xffffffffu, (m0 | m1) != 0u)) {
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (m0 == 0u) { m0 = m1; m1 = 0u; base += 32; }
+                if (m0 != 0u) {
+                    const int ent = __float_as_int(sh.f[base + __ffs(m0) - 1].w);
+                    m0 &= m0 - 1u;
+                    if (ent != self_e) {
+                        sh.ring[cnt & (NB_RING - 1)][lane] = ent;
+                        cnt++;
+                    }
+                }
+            }
+            if (half == 0 && !__any_sync(0xffffffffu, (m0 | m1) != 0u)) break;
+        }
+        if (cnt - out >= 8) {
+            if (out < maxn) write_sector(sh, lane, row, out);
+            out += 8;
+        }
     }
 }
 
@@ -307,6 +340,8 @@ __device__ uint32_t build_cell(const CellSys &y, int c, BuildShared<POLY, TILE> 
         const float by0 = warp_min(yif), by1 = warp_max(yif);
         const float bz0 = warp_min(zif), bz1 = warp_max(zif);
         int cnt = 0, nb = 0;  // the owner lane's list and bond counts
+        int out = 0;          // entries already in the row: whole sectors
+        int32_t *const row = TILE ? nullptr : y.nbr + nb_row(i, maxn);
         uint16_t *const row16 = TILE ? y.nbr16 + tile_row16(i, maxn) : nullptr;
         const int self_e = i | (NB_NOSHIFT << NB_SHIFT_BITS);  // the owner's own entry
         const int nown = min(32, ccount - pass * 32);
@@ -319,19 +354,19 @@ __device__ uint32_t build_cell(const CellSys &y, int c, BuildShared<POLY, TILE> 
             sh.ochain[lane] = own ? y.chain[i] : -1;
             sh.obf[lane] = own ? y.bflag[i] : make_int4(0, 0, 0, 0);
         }
-        for (int base = 0; base < total; base += NB_STAGE) {
-            const int take = min(NB_STAGE, total - base);
+        // Candidates are staged 32 a step, in visiting order; those that cannot
+        // lie within rneighbr of some owner of this pass are left out (ballot
+        // compaction). Whenever 64 are there, and at the end, the owners test
+        // them and append their hits; what is left over moves to the front.
+        int kept = 0;
+        for (int t0 = 0; t0 < total; t0 += 32) {
             __syncwarp();
-            // stage the window's candidates that can lie within rneighbr of
-            // some owner of this pass, in visiting order (ballot compaction)
-            int kept = 0;
-            for (int t0 = 0; t0 < take; t0 += 32) {
-                const int t = t0 + lane;
+            {
+                const int q = t0 + lane;
                 bool keep = false;
                 float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
                 int j = 0, loc = 0;
-                if (t < take) {
-                    const int q = base + t;
+                if (q < total) {
                     int k = 0;  // segment containing q: largest k with off[k] <= q
 #pragma unroll
                     for (int step = 32; step > 0; step >>= 1)
@@ -362,96 +397,117 @@ __device__ uint32_t build_cell(const CellSys &y, int c, BuildShared<POLY, TILE> 
                 kept += __popc(m);
             }
             __syncwarp();
-            // lane = candidate, loop over owners
-            for (int t0 = 0; t0 < kept; t0 += 32) {
-                const int cq = t0 + lane;
-                const bool valid = cq < kept;
-                // candidate sentinel on the other side: r^2 = inf against every owner
-                const float4 f = valid ? sh.f[cq] : make_float4(-1e30f, -1e30f, -1e30f, 0.f);
-                const int e = __float_as_int(f.w);
-                const unsigned long long fx2 = pack_f32x2(f.x, f.x), fy2 = pack_f32x2(f.y, f.y),
-                                         fz2 = pack_f32x2(f.z, f.z);
-                int2 cs = make_int2(-2, 0);
-                if (POLY && valid) cs = sh.cs[cq];
-                unsigned mine_reg = 0u;  // polymers: the owner lane keeps its ballot in a register
-                // owners in groups of NB_OG (pairs in packed FP32): independent chains
-                // for the scheduler
-                for (int o0 = 0; o0 < nown; o0 += NB_OG) {
-                    bool hit[NB_OG], exact[NB_OG];
-                    float r2f[NB_OG];
-                    bool anyx = false;
+            if (kept < 64 && t0 + 32 < total) continue;
+            do {
+                unsigned mine[2] = {0u, 0u};  // the owner lane's hits among the two halves
+#pragma unroll 1
+                for (int half = 0; 32 * half < min(kept, 64); half++) {
+                    const int cq = 32 * half + lane;
+                    const bool valid = cq < kept;
+                    // candidate sentinel on the other side: r^2 = inf against every owner
+                    const float4 f = valid ? sh.f[cq] : make_float4(-1e30f, -1e30f, -1e30f, 0.f);
+                    const int e = __float_as_int(f.w);
+                    const unsigned long long fx2 = pack_f32x2(f.x, f.x), fy2 = pack_f32x2(f.y, f.y),
+                                             fz2 = pack_f32x2(f.z, f.z);
+                    int2 cs = make_int2(-2, 0);
+                    if (POLY && valid) cs = sh.cs[cq];
+                    unsigned mine_reg = 0u;  // polymers: the owner lane keeps its ballot in a register
+                    // owners in groups of NB_OG (pairs in packed FP32): independent chains
+                    // for the scheduler
+                    for (int o0 = 0; o0 < nown; o0 += NB_OG) {
+                        bool hit[NB_OG], exact[NB_OG];
+                        float r2f[NB_OG];
+                        bool anyx = false;
 #pragma unroll
-                    for (int h = 0; h < NB_OG; h += 2) {
-                        const unsigned long long dx = sub_f32x2(lds_f32x2(&sh.ox[o0 + h]), fx2);
-                        const unsigned long long dy = sub_f32x2(lds_f32x2(&sh.oy[o0 + h]), fy2);
-                        const unsigned long long dz = sub_f32x2(lds_f32x2(&sh.oz[o0 + h]), fz2);
-                        const unsigned long long t = fma_f32x2(dz, dz, fma_f32x2(dy, dy, mul_f32x2(dx, dx)));
-                        r2f[h] = __uint_as_float((unsigned)t);
-                        r2f[h + 1] = __uint_as_float((unsigned)(t >> 32));
-                    }
-#pragma unroll
-                    for (int u = 0; u < NB_OG; u++) {
-                        // the band around rneighbr2 is decided in FP64; the owner
-                        // itself (r2f exactly 0) is a hit here, dropped at the append
-                        hit[u] = r2f[u] < lo32 && (!POLY || r2f[u] > 0.f);
-                        exact[u] = !hit[u] && r2f[u] <= hi32;
-                        anyx |= exact[u];
-                    }
-                    if (__any_sync(0xffffffffu, anyx)) {
-#pragma unroll
-                        for (int u = 0; u < NB_OG; u++)
-                            if (exact[u]) hit[u] = exact_pair(P, sh.oi[o0 + u], e, y.L, y.rn2);
-                    }
-#pragma unroll
-                    for (int u = 0; u < NB_OG; u++) {
-                        const unsigned m = __ballot_sync(0xffffffffu, hit[u]);
-                        if (POLY) {
-                            if (lane == o0 + u) mine_reg = m;
-                        } else if (lane == 0) {
-                            sh.hits[o0 + u] = m;
+                        for (int h = 0; h < NB_OG; h += 2) {
+                            const unsigned long long dx = sub_f32x2(lds_f32x2(&sh.ox[o0 + h]), fx2);
+                            const unsigned long long dy = sub_f32x2(lds_f32x2(&sh.oy[o0 + h]), fy2);
+                            const unsigned long long dz = sub_f32x2(lds_f32x2(&sh.oz[o0 + h]), fz2);
+                            const unsigned long long t = fma_f32x2(dz, dz, fma_f32x2(dy, dy, mul_f32x2(dx, dx)));
+                            r2f[h] = __uint_as_float((unsigned)t);
+                            r2f[h + 1] = __uint_as_float((unsigned)(t >> 32));
                         }
-                    }
-                    if (POLY) {
-                        int addb = 0;
 #pragma unroll
                         for (int u = 0; u < NB_OG; u++) {
-                            bool bond = false;
-                            if (valid && o0 + u < nown && cs.x == sh.ochain[o0 + u] &&
-                                !((e & NB_INDEX_MASK) == sh.oi[o0 + u] && (e >> NB_SHIFT_BITS) == NB_NOSHIFT)) {
-                                const int pos = cs.y - 1, grp = pos / 31, ex = pos % 31;
-                                const int4 bf = sh.obf[o0 + u];
-                                const int word = grp == 0 ? bf.x : grp == 1 ? bf.y : grp == 2 ? bf.z : bf.w;
-                                bond = pos >= 0 && grp < 4 && ((word >> ex) & 1);
-                            }
-                            const unsigned mb = __ballot_sync(0xffffffffu, bond);
-                            const int b0 = __shfl_sync(0xffffffffu, nb, o0 + u);
-                            if (bond) {
-                                const int k = b0 + __popc(mb & lt);
-                                if (k < 4) y.bnd[(size_t)sh.oi[o0 + u] * 4 + k] = e;
-                            }
-                            if (lane == o0 + u) addb = __popc(mb);
+                            // the band around rneighbr2 is decided in FP64; the owner
+                            // itself (r2f exactly 0) is a hit here, dropped at the append
+                            hit[u] = r2f[u] < lo32 && (!POLY || r2f[u] > 0.f);
+                            exact[u] = !hit[u] && r2f[u] <= hi32;
+                            anyx |= exact[u];
                         }
-                        nb += addb;
+                        if (__any_sync(0xffffffffu, anyx)) {
+#pragma unroll
+                            for (int u = 0; u < NB_OG; u++)
+                                if (exact[u]) hit[u] = exact_pair(P, sh.oi[o0 + u], e, y.L, y.rn2);
+                        }
+#pragma unroll
+                        for (int u = 0; u < NB_OG; u++) {
+                            const unsigned m = __ballot_sync(0xffffffffu, hit[u]);
+                            if (POLY) {
+                                if (lane == o0 + u) mine_reg = m;
+                            } else if (lane == 0) {
+                                sh.hits[half][o0 + u] = m;
+                            }
+                        }
+                        if (POLY) {
+                            int addb = 0;
+#pragma unroll
+                            for (int u = 0; u < NB_OG; u++) {
+                                bool bond = false;
+                                if (valid && o0 + u < nown && cs.x == sh.ochain[o0 + u] &&
+                                    !((e & NB_INDEX_MASK) == sh.oi[o0 + u] && (e >> NB_SHIFT_BITS) == NB_NOSHIFT)) {
+                                    const int pos = cs.y - 1, grp = pos / 31, ex = pos % 31;
+                                    const int4 bf = sh.obf[o0 + u];
+                                    const int word = grp == 0 ? bf.x : grp == 1 ? bf.y : grp == 2 ? bf.z : bf.w;
+                                    bond = pos >= 0 && grp < 4 && ((word >> ex) & 1);
+                                }
+                                const unsigned mb = __ballot_sync(0xffffffffu, bond);
+                                const int b0 = __shfl_sync(0xffffffffu, nb, o0 + u);
+                                if (bond) {
+                                    const int k = b0 + __popc(mb & lt);
+                                    if (k < 4) y.bnd[(size_t)sh.oi[o0 + u] * 4 + k] = e;
+                                }
+                                if (lane == o0 + u) addb = __popc(mb);
+                            }
+                            nb += addb;
+                        }
                     }
+                    if (POLY) mine[half] = mine_reg;
                 }
-                // the owner lane appends its hits in candidate order, all but
-                // itself, through its chunk buffer (whole sectors to the row)
-                if (!POLY) __syncwarp();
-                unsigned mine_hits = POLY ? mine_reg : (lane < nown ? sh.hits[lane] : 0u);
-                while (mine_hits) {
-                    const int b = __ffs(mine_hits) - 1;
-                    mine_hits &= mine_hits - 1u;
-                    const int ent = __float_as_int(sh.f[t0 + b].w);
-                    if (POLY || ent != self_e) {
-                        if (cnt < maxn) append_entry<TILE>(sh, lane, y.tT, y.nbr, row16, i, maxn, cnt, ent,
-                                                           TILE ? sh.loc[t0 + b] : (unsigned short)0);
-                        cnt++;
+                if (!POLY) {
+                    __syncwarp();
+                    mine[0] = lane < nown && kept > 0 ? sh.hits[0][lane] : 0u;
+                    mine[1] = lane < nown && kept > 32 ? sh.hits[1][lane] : 0u;
+                }
+                if constexpr (TILE) {
+                    for (int half = 0; half < 2; half++)
+                        for (unsigned m = mine[half]; m != 0u; m &= m - 1u) {
+                            const int b = 32 * half + __ffs(m) - 1;
+                            if (__float_as_int(sh.f[b].w) == self_e) continue;
+                            if (cnt < maxn) append_tile(sh, lane, y.tT, row16, cnt, sh.loc[b]);
+                            cnt++;
+                        }
+                } else {
+                    append_hits(sh, lane, mine[0], mine[1], self_e, row, maxn, cnt, out);
+                }
+                __syncwarp();
+                const int left = kept - 64;  // below 32: a step adds at most that many
+                if (left > 0) {
+                    if (lane < left) {
+                        sh.f[lane] = sh.f[64 + lane];
+                        if (TILE) sh.loc[lane] = sh.loc[64 + lane];
+                        if (POLY) sh.cs[lane] = sh.cs[64 + lane];
                     }
+                    __syncwarp();
                 }
-                if (!POLY) __syncwarp();
-            }
+                kept = max(left, 0);
+            } while (kept > 0 && t0 + 32 >= total);
         }
-        if (own && cnt < maxn) flush_entries<TILE>(sh, lane, y.tT, y.nbr, row16, i, maxn, cnt, y.tdummy);
+        if constexpr (TILE) {
+            if (own && cnt < maxn) flush_tile(sh, lane, y.tT, row16, cnt, y.tdummy);
+        } else if (cnt > out && out < maxn) {  // the last, partial sector lies inside the row
+            write_sector(sh, lane, row, out);
+        }
         if (own) {
             y.nnbr[i] = cnt < maxn ? cnt : maxn;
             atomicMax(y.max_nbr, cnt);
@@ -492,13 +548,13 @@ struct BlockShared {
     int start[NB_BSEG], code[NB_BSEG];
     int lbase[TILE ? NB_BSEG : 1];               // segment k's first candidate in the block staging
     unsigned short loc[TILE ? NB_STAGE : 1];     // staged candidates' staging offsets
-    alignas(16) int ob[TILE ? 1 : 32][8];        // owner lane's chunk being filled (generic rows)
+    int ring[TILE ? 1 : NB_RING][32];            // entries an owner lane has not written yet (generic rows)
     alignas(16) unsigned short ob16[TILE ? 32 : 1][32];  // (tiled rows, 4 T <= 32 entries)
     unsigned char segallow[NB_BSEG];
     int opre[9], ostart[8];         // owners by block cell: prefix counts, first molecule
     int ochain[POLY ? 32 : 1];
     alignas(16) int4 obf[POLY ? 32 : 1];
-    unsigned hits[POLY ? 1 : 32];   // per owner: which of the 32 candidates hit (polymers: registers)
+    unsigned hits[POLY ? 1 : 2][32];  // per owner: which of the 32 candidates hit (polymers: registers)
 };
 
 template <bool POLY, bool TILE = false>
@@ -638,7 +694,8 @@ __device__ uint32_t build_block(const CellSys &y, int blk, BlockShared<POLY, TIL
         const float bx_lo = warp_min(own ? xif : 3e38f), bx_hi = warp_max(own ? xif : -3e38f);
         const float by_lo = warp_min(own ? yif : 3e38f), by_hi = warp_max(own ? yif : -3e38f);
         const float bz_lo = warp_min(own ? zif : 3e38f), bz_hi = warp_max(own ? zif : -3e38f);
-        int cnt = 0, nb = 0;
+        int cnt = 0, nb = 0, out = 0;
+        int32_t *const row = TILE ? nullptr : y.nbr + nb_row(i, maxn);
         uint16_t *const row16 = TILE ? y.nbr16 + tile_row16(i, maxn) : nullptr;
         const int self_e = i | (NB_NOSHIFT << NB_SHIFT_BITS);  // the owner's own entry
         const int nown = min(32, nowners - pass * 32);
@@ -652,18 +709,20 @@ __device__ uint32_t build_block(const CellSys &y, int blk, BlockShared<POLY, TIL
             sh.ochain[lane] = own ? y.chain[i] : -1;
             sh.obf[lane] = own ? y.bflag[i] : make_int4(0, 0, 0, 0);
         }
-        for (int base = 0; base < total; base += NB_STAGE) {
-            const int take = min(NB_STAGE, total - base);
+        // Candidates are staged 32 a step, in visiting order; those that cannot
+        // lie within rneighbr of some owner of this pass are left out (ballot
+        // compaction). Whenever 64 are there, and at the end, the owners test
+        // them and append their hits; what is left over moves to the front.
+        int kept = 0;
+        for (int t0 = 0; t0 < total; t0 += 32) {
             __syncwarp();
-            int kept = 0;
-            for (int t0 = 0; t0 < take; t0 += 32) {
-                const int t = t0 + lane;
+            {
+                const int q = t0 + lane;
                 bool keep = false;
                 float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
                 unsigned al = 0u;
                 int j = 0, loc = 0;
-                if (t < take) {
-                    const int q = base + t;
+                if (q < total) {
                     int kk = 0;  // segment containing q: largest kk with off[kk] <= q
 #pragma unroll
                     for (int step = 64; step > 0; step >>= 1)
@@ -694,93 +753,116 @@ __device__ uint32_t build_block(const CellSys &y, int blk, BlockShared<POLY, TIL
                 kept += __popc(m);
             }
             __syncwarp();
-            for (int t0 = 0; t0 < kept; t0 += 32) {
-                const int cq = t0 + lane;
-                const bool valid = cq < kept;
-                const float4 f = valid ? sh.f[cq] : make_float4(-1e30f, -1e30f, -1e30f, 0.f);
-                const unsigned callow = valid ? sh.allow[cq] : 0u;
-                const int e = __float_as_int(f.w);
-                const unsigned long long fx2 = pack_f32x2(f.x, f.x), fy2 = pack_f32x2(f.y, f.y),
-                                         fz2 = pack_f32x2(f.z, f.z);
-                int2 cs = make_int2(-2, 0);
-                if (POLY && valid) cs = sh.cs[cq];
-                unsigned mine_reg = 0u;  // polymers: the owner lane keeps its ballot in a register
-                for (int o0 = 0; o0 < nown; o0 += NB_OG) {
-                    bool hit[NB_OG], exact[NB_OG];
-                    float r2f[NB_OG];
-                    bool anyx = false;
+            if (kept < 64 && t0 + 32 < total) continue;
+            do {
+                unsigned mine[2] = {0u, 0u};  // the owner lane's hits among the two halves
+#pragma unroll 1
+                for (int half = 0; 32 * half < min(kept, 64); half++) {
+                    const int cq = 32 * half + lane;
+                    const bool valid = cq < kept;
+                    const float4 f = valid ? sh.f[cq] : make_float4(-1e30f, -1e30f, -1e30f, 0.f);
+                    const unsigned callow = valid ? sh.allow[cq] : 0u;
+                    const int e = __float_as_int(f.w);
+                    const unsigned long long fx2 = pack_f32x2(f.x, f.x), fy2 = pack_f32x2(f.y, f.y),
+                                             fz2 = pack_f32x2(f.z, f.z);
+                    int2 cs = make_int2(-2, 0);
+                    if (POLY && valid) cs = sh.cs[cq];
+                    unsigned mine_reg = 0u;  // polymers: the owner lane keeps its ballot in a register
+                    for (int o0 = 0; o0 < nown; o0 += NB_OG) {
+                        bool hit[NB_OG], exact[NB_OG];
+                        float r2f[NB_OG];
+                        bool anyx = false;
 #pragma unroll
-                    for (int h = 0; h < NB_OG; h += 2) {
-                        const unsigned long long dx = sub_f32x2(lds_f32x2(&sh.ox[o0 + h]), fx2);
-                        const unsigned long long dy = sub_f32x2(lds_f32x2(&sh.oy[o0 + h]), fy2);
-                        const unsigned long long dz = sub_f32x2(lds_f32x2(&sh.oz[o0 + h]), fz2);
-                        const unsigned long long t = fma_f32x2(dz, dz, fma_f32x2(dy, dy, mul_f32x2(dx, dx)));
-                        r2f[h] = __uint_as_float((unsigned)t);
-                        r2f[h + 1] = __uint_as_float((unsigned)(t >> 32));
-                    }
-#pragma unroll
-                    for (int u = 0; u < NB_OG; u++) {
-                        const bool ok = (callow & sh.oallow[o0 + u]) != 0u;
-                        // the owner itself: dropped at the append (polymers: decided in FP64)
-                        hit[u] = ok && r2f[u] < lo32 && (!POLY || r2f[u] > 0.f);
-                        exact[u] = ok && !hit[u] && r2f[u] <= hi32;
-                        anyx |= exact[u];
-                    }
-                    if (__any_sync(0xffffffffu, anyx)) {
-#pragma unroll
-                        for (int u = 0; u < NB_OG; u++)
-                            if (exact[u]) hit[u] = exact_pair(P, sh.oi[o0 + u], e, y.L, y.rn2);
-                    }
-#pragma unroll
-                    for (int u = 0; u < NB_OG; u++) {
-                        const unsigned m = __ballot_sync(0xffffffffu, hit[u]);
-                        if (POLY) {
-                            if (lane == o0 + u) mine_reg = m;
-                        } else if (lane == 0) {
-                            sh.hits[o0 + u] = m;
+                        for (int h = 0; h < NB_OG; h += 2) {
+                            const unsigned long long dx = sub_f32x2(lds_f32x2(&sh.ox[o0 + h]), fx2);
+                            const unsigned long long dy = sub_f32x2(lds_f32x2(&sh.oy[o0 + h]), fy2);
+                            const unsigned long long dz = sub_f32x2(lds_f32x2(&sh.oz[o0 + h]), fz2);
+                            const unsigned long long t = fma_f32x2(dz, dz, fma_f32x2(dy, dy, mul_f32x2(dx, dx)));
+                            r2f[h] = __uint_as_float((unsigned)t);
+                            r2f[h + 1] = __uint_as_float((unsigned)(t >> 32));
                         }
-                    }
-                    if (POLY) {
-                        int addb = 0;
 #pragma unroll
                         for (int u = 0; u < NB_OG; u++) {
-                            bool bond = false;
-                            if ((callow & sh.oallow[o0 + u]) != 0u && cs.x == sh.ochain[o0 + u] &&
-                                !((e & NB_INDEX_MASK) == sh.oi[o0 + u] && (e >> NB_SHIFT_BITS) == NB_NOSHIFT)) {
-                                const int pos = cs.y - 1, grp = pos / 31, ex = pos % 31;
-                                const int4 bf = sh.obf[o0 + u];
-                                const int word = grp == 0 ? bf.x : grp == 1 ? bf.y : grp == 2 ? bf.z : bf.w;
-                                bond = pos >= 0 && grp < 4 && ((word >> ex) & 1);
-                            }
-                            const unsigned mb = __ballot_sync(0xffffffffu, bond);
-                            const int b0 = __shfl_sync(0xffffffffu, nb, o0 + u);
-                            if (bond) {
-                                const int kb = b0 + __popc(mb & lt);
-                                if (kb < 4) y.bnd[(size_t)sh.oi[o0 + u] * 4 + kb] = e;
-                            }
-                            if (lane == o0 + u) addb = __popc(mb);
+                            const bool ok = (callow & sh.oallow[o0 + u]) != 0u;
+                            // the owner itself: dropped at the append (polymers: decided in FP64)
+                            hit[u] = ok && r2f[u] < lo32 && (!POLY || r2f[u] > 0.f);
+                            exact[u] = ok && !hit[u] && r2f[u] <= hi32;
+                            anyx |= exact[u];
                         }
-                        nb += addb;
+                        if (__any_sync(0xffffffffu, anyx)) {
+#pragma unroll
+                            for (int u = 0; u < NB_OG; u++)
+                                if (exact[u]) hit[u] = exact_pair(P, sh.oi[o0 + u], e, y.L, y.rn2);
+                        }
+#pragma unroll
+                        for (int u = 0; u < NB_OG; u++) {
+                            const unsigned m = __ballot_sync(0xffffffffu, hit[u]);
+                            if (POLY) {
+                                if (lane == o0 + u) mine_reg = m;
+                            } else if (lane == 0) {
+                                sh.hits[half][o0 + u] = m;
+                            }
+                        }
+                        if (POLY) {
+                            int addb = 0;
+#pragma unroll
+                            for (int u = 0; u < NB_OG; u++) {
+                                bool bond = false;
+                                if ((callow & sh.oallow[o0 + u]) != 0u && cs.x == sh.ochain[o0 + u] &&
+                                    !((e & NB_INDEX_MASK) == sh.oi[o0 + u] && (e >> NB_SHIFT_BITS) == NB_NOSHIFT)) {
+                                    const int pos = cs.y - 1, grp = pos / 31, ex = pos % 31;
+                                    const int4 bf = sh.obf[o0 + u];
+                                    const int word = grp == 0 ? bf.x : grp == 1 ? bf.y : grp == 2 ? bf.z : bf.w;
+                                    bond = pos >= 0 && grp < 4 && ((word >> ex) & 1);
+                                }
+                                const unsigned mb = __ballot_sync(0xffffffffu, bond);
+                                const int b0 = __shfl_sync(0xffffffffu, nb, o0 + u);
+                                if (bond) {
+                                    const int kb = b0 + __popc(mb & lt);
+                                    if (kb < 4) y.bnd[(size_t)sh.oi[o0 + u] * 4 + kb] = e;
+                                }
+                                if (lane == o0 + u) addb = __popc(mb);
+                            }
+                            nb += addb;
+                        }
                     }
+                    if (POLY) mine[half] = mine_reg;
                 }
-                // the owner lane appends its hits in candidate order, all but
-                // itself, through its chunk buffer (whole sectors to the row)
-                if (!POLY) __syncwarp();
-                unsigned mine_hits = POLY ? mine_reg : (lane < nown ? sh.hits[lane] : 0u);
-                while (mine_hits) {
-                    const int b = __ffs(mine_hits) - 1;
-                    mine_hits &= mine_hits - 1u;
-                    const int ent = __float_as_int(sh.f[t0 + b].w);
-                    if (POLY || ent != self_e) {
-                        if (cnt < maxn) append_entry<TILE>(sh, lane, y.tT, y.nbr, row16, i, maxn, cnt, ent,
-                                                           TILE ? sh.loc[t0 + b] : (unsigned short)0);
-                        cnt++;
+                if (!POLY) {
+                    __syncwarp();
+                    mine[0] = lane < nown && kept > 0 ? sh.hits[0][lane] : 0u;
+                    mine[1] = lane < nown && kept > 32 ? sh.hits[1][lane] : 0u;
+                }
+                if constexpr (TILE) {
+                    for (int half = 0; half < 2; half++)
+                        for (unsigned m = mine[half]; m != 0u; m &= m - 1u) {
+                            const int b = 32 * half + __ffs(m) - 1;
+                            if (__float_as_int(sh.f[b].w) == self_e) continue;
+                            if (cnt < maxn) append_tile(sh, lane, y.tT, row16, cnt, sh.loc[b]);
+                            cnt++;
+                        }
+                } else {
+                    append_hits(sh, lane, mine[0], mine[1], self_e, row, maxn, cnt, out);
+                }
+                __syncwarp();
+                const int left = kept - 64;  // below 32: a step adds at most that many
+                if (left > 0) {
+                    if (lane < left) {
+                        sh.f[lane] = sh.f[64 + lane];
+                        sh.allow[lane] = sh.allow[64 + lane];
+                        if (TILE) sh.loc[lane] = sh.loc[64 + lane];
+                        if (POLY) sh.cs[lane] = sh.cs[64 + lane];
                     }
+                    __syncwarp();
                 }
-                if (!POLY) __syncwarp();
-            }
+                kept = max(left, 0);
+            } while (kept > 0 && t0 + 32 >= total);
         }
-        if (own && cnt < maxn) flush_entries<TILE>(sh, lane, y.tT, y.nbr, row16, i, maxn, cnt, y.tdummy);
+        if constexpr (TILE) {
+            if (own && cnt < maxn) flush_tile(sh, lane, y.tT, row16, cnt, y.tdummy);
+        } else if (cnt > out && out < maxn) {  // the last, partial sector lies inside the row
+            write_sector(sh, lane, row, out);
+        }
         if (own) {
             y.nnbr[i] = cnt < maxn ? cnt : maxn;
             atomicMax(y.max_nbr, cnt);

@@ -42,6 +42,7 @@ struct FmScalars {
     int32_t pcount;           // samples in pacc
     int32_t tile_next;        // tiled force kernel: next block to hand out (the last taker resets it)
     int32_t umax;             // tiled path: largest staged neighbourhood seen at the last build
+    int32_t strays;           // last cell sort: a real molecule is binned in a halo cell
     int32_t g_iter;           // rebuild graph: iteration its next decision is for
     int32_t cur_iter;         // rebuild graph: iteration of the last decision (errors in its body)
     int64_t graph_kernels;    // rebuild graph: kernels its conditional body has run
@@ -102,7 +103,7 @@ struct FmDev {
     // reorder scratch
     double *tvx, *tvy, *tvz, *tax, *tay, *taz;
     // cells (extended grid, x fastest)
-    int32_t *cell_of;      // per molecule (old order) cell id
+    int32_t *cell_of;      // per molecule cell id: by old slot until the cell sort, by new slot after it
     int32_t *cell_count;   // ncell
     int32_t *cell_start;   // ncell + 1
     int32_t *perm;         // new slot -> old slot
@@ -124,7 +125,8 @@ struct FmDev {
     int32_t *bnd, *nbond;
     // Mie_potential 1: per-type-pair constants, per-type masses; a molecule's
     // type (1-based) rides in the w component of its position
-    int build_blocks;            // list build: one warp per 2x2x2 cells (sparse systems)
+    int build_rows;              // list build by molecule (fm_rows.cuh); else by warp, build_blocks choosing
+    int build_blocks;            // one warp per 2x2x2 cells (sparse systems) or per cell
     // Tiled force path (tile = 1): the extended cell grid is cut into blocks of
     // 2x2x2 cells; the force kernel stages the positions of a block's 4x4x4
     // cell neighbourhood (images applied) in shared memory, and list entries
@@ -186,20 +188,26 @@ __host__ __device__ inline double4 *cur_pos(const FmDev &d, int pset) { return p
 constexpr int NB_SHIFT_BITS = 26;
 constexpr int32_t NB_INDEX_MASK = (1 << NB_SHIFT_BITS) - 1;
 constexpr int MAX_MOLECULES = NB_INDEX_MASK;
+constexpr int NB_NOSHIFT = 1 | (1 << 2) | (1 << 4);  // image code of an unshifted partner
 
 // Neighbour list layout: molecules in groups of 32, each molecule's entries
 // in chunks of 8 (one 32-byte sector); chunk c of the 32 molecules of a group
-// is one contiguous 1 KB block (molecule i%32 at offset 32 (i%32) bytes), so a
-// warp that reads a 16-byte half of chunk c of its 32 molecules reads 32
-// sectors of one block, and the list build writes each sector whole (a
-// sector shared by two molecules written at different times would reach
-// DRAM half-written once the list outgrows L2).  The array holds
-// ceil(n/32)*32 rows of maxn (a multiple of 8) entries.
+// is one contiguous 1 KB block (molecule i%32 at offset 32 (i%32) bytes), and
+// the list build writes each sector whole (a sector shared by two molecules
+// written at different times would reach DRAM half-written once the list
+// outgrows L2). In a chunk entry k is at place 2 (k % 4) + (k / 4) % 2: four
+// lanes that read 8 bytes each get entries k .. k+3 in one register and
+// k+4 .. k+7 in the next, so their gathers are of neighbouring entries
+// (row_entries, fm_device.cuh).  The array holds ceil(n/32)*32 rows of maxn
+// (a multiple of 8) entries.
 __host__ __device__ inline size_t nb_row(int i, int maxn)
 {
     return (size_t)(i >> 5) * (size_t)maxn * 32u + (size_t)(i & 31) * 8u;
 }
-__host__ __device__ inline size_t nb_col(int k) { return (size_t)(k & ~7) * 32u + (size_t)(k & 7); }
+__host__ __device__ inline size_t nb_col(int k)
+{
+    return (size_t)(k & ~7) * 32u + (size_t)((k & 3) * 2 + ((k >> 2) & 1));
+}
 inline size_t nb_rows(int n) { return ((size_t)n + 31u) / 32u * 32u; }
 
 // Subdomain bookkeeping of the decomposition kernels (fm_dd_kernels.cu).
@@ -250,6 +258,10 @@ void launch_scan_cells(const FmDev &d, int gated, cudaStream_t st);
 void launch_scatter(const FmDev &d, int gated, cudaStream_t st);
 void launch_reorder(const FmDev &d, int gated, double4 *tpos, int32_t *tuidx, cudaStream_t st);
 void launch_build_nlist(const FmDev &d, int gated, int iter, cudaStream_t st);
+// The same rows by molecule (fm_rows.cu), for up to ROWS_MAX_MOLECULES: 32,000
+// molecules 78 us against ~130 by warp, 108,000 264 against 160.
+constexpr int ROWS_MAX_MOLECULES = 65536;
+void launch_rows(const FmDev &d, int gated, int iter, cudaStream_t st);
 // angular_potential: orders each middle bead's two bonds as the reference's
 // list build discovers them (after every build).
 void launch_angular_order(const FmDev &d, int gated, int iter, cudaStream_t st);
@@ -264,6 +276,8 @@ void launch_tile_to_generic(const FmDev &d, int32_t *out, int maxn, cudaStream_t
 // Forces: mode 0 forces only, 1 forces + move(2), 2 forces + move(2) + next
 // move(1), 3 forces + leap-frog move.
 void launch_force(const FmDev &d, int record, int mode, int tpm, cudaStream_t st);
+void launch_force_lj(const FmDev &d, int record, int mode, int tpm, cudaStream_t st);     // fm_force_lj.cu
+void launch_force_types(const FmDev &d, int record, int mode, int tpm, cudaStream_t st);  // fm_force_types.cu
 void launch_record(const FmDev &d, int iter, double simtime, cudaStream_t st);
 void launch_all_pairs(const FmDev &d, int record, int mode, cudaStream_t st);
 // Record partials straight from the per-molecule arrays (PE, virial) and the

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fm_common.cuh"
+
 namespace fm {
 
 // |v|^2 in the reference's dot_product order, no contraction.
@@ -75,6 +77,49 @@ __device__ __forceinline__ int4 ld_stream_int4(const int4 *p)
     return r;
 }
 
+__device__ __forceinline__ int2 ld_stream_int2(const int2 *p)
+{
+    int2 r;
+    asm("ld.global.nc.L1::no_allocate.v2.s32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
+    return r;
+}
+
+// Step s of lane `lane` of the TPM lanes that walk a row of cnt entries: four
+// entries, of which number q counts while row_left > row_off(q). The lanes of a
+// molecule take neighbouring entries, and slots ascend along a row, so a
+// warp's gather of 32 partners meets fewer lines, of which L1 serves one a
+// clock: by count over a 1M liquid's rows 21 with one lane a molecule and 13
+// with four. row_first is the first entry of a step.
+template <int TPM>
+__device__ __forceinline__ int row_first(int s)
+{
+    return TPM == 1 ? 8 * (s >> 1) + 2 * (s & 1) : 4 * TPM * s;
+}
+template <int TPM>
+__device__ __forceinline__ int row_left(int s, int lane, int cnt)
+{
+    return cnt - (TPM <= 2 ? row_first<TPM>(s) + 2 * lane : 4 * TPM * s + 8 * (lane >> 2) + (lane & 3));
+}
+template <int TPM>
+__host__ __device__ constexpr int row_off(int q)
+{
+    return TPM <= 2 ? (q & 1) * 4 + (q >> 1) : (q >> 1) * 2 * TPM + (q & 1) * 4;
+}
+template <int TPM>
+__device__ __forceinline__ int4 row_entries(const int32_t *L, int s, int lane, int left)
+{
+    if (TPM <= 2) {  // half a chunk: entries h, h + 4, h + 1, h + 5
+        return ld_stream_int4(reinterpret_cast<const int4 *>(
+            L + (TPM == 1 ? (size_t)(s >> 1) * 256u + 4 * (s & 1) : (size_t)s * 256u + 4 * lane)));
+    }
+    // entries t and t + 4 of two chunks
+    const int32_t *p = L + (size_t)((TPM / 2) * s + (lane >> 2)) * 256u + 2 * (lane & 3);
+    int2 a = make_int2(0, 0), b = make_int2(0, 0);
+    if (left > 0) a = ld_stream_int2(reinterpret_cast<const int2 *>(p));
+    if (left > row_off<TPM>(2)) b = ld_stream_int2(reinterpret_cast<const int2 *>(p + (TPM / 4) * 256));
+    return make_int4(a.x, a.y, b.x, b.y);
+}
+
 // FP32 reciprocal of the precision form's pair magnitudes (s = 1/r^2): the
 // hardware's approximate reciprocal (rcp.approx.ftz.f32, about 1 ulp; r^2 is
 // never subnormal here), one instruction where a correctly rounded
@@ -138,6 +183,20 @@ __device__ __forceinline__ int bin_axis(double x, double hd, double cs, int ne, 
     int c = __double2int_ru(q);  // round toward +inf == ceiling for in-range values
     if (c < 0 || c > ne - 1) { bad = true; c = c < 0 ? 0 : ne - 1; }
     return c;
+}
+
+// Octant of extended cell (cx, cy, cz) that p lies in, x fastest. The
+// line between two halves lies 2^-20 of a cell before their middle, so that a
+// lattice site exactly in the middle falls in the same half whatever box of
+// the periodic system its coordinate is rounded in.
+__device__ __forceinline__ int sub_cell(const double4 &p, int cx, int cy, int cz, const double (&hd)[3],
+                                        const double (&cs)[3])
+{
+    const float x = (float)((p.x + hd[0]) - (cx - 0.5) * cs[0]), y = (float)((p.y + hd[1]) - (cy - 0.5) * cs[1]);
+    const float z = (float)((p.z + hd[2]) - (cz - 0.5) * cs[2]);
+    const float tx = (float)cs[0] * -9.5367431640625e-7f, ty = (float)cs[1] * -9.5367431640625e-7f;
+    const float tz = (float)cs[2] * -9.5367431640625e-7f;
+    return (x > tx ? 1 : 0) | (y > ty ? 2 : 0) | (z > tz ? 4 : 0);
 }
 
 __device__ __forceinline__ bool is_halo(int x, int ne) { return x == 0 || x == ne - 1; }

@@ -586,16 +586,17 @@ __global__ void __launch_bounds__(EF_THREADS, REC ? 2 : 4) k_e_force(EngDev d)
             const int cnt = d.nnbr[i];
             const int32_t *L = d.nbr + s.list_off + nb_row(i - s.mol_off, s.maxn);
             const double4 *Pj = P + s.mol_off;
-            for (int k0 = lane * 4; k0 < cnt; k0 += 4 * TPM) {
-                const int4 e4 = ld_stream_int4(reinterpret_cast<const int4 *>(L + nb_col(k0)));
+            for (int st = 0; row_first<TPM>(st) < cnt; st++) {
+                const int left = row_left<TPM>(st, lane, cnt);
+                const int4 e4 = row_entries<TPM>(L, st, lane, left);
                 const int ev[4] = {e4.x, e4.y, e4.z, e4.w};
                 double4 pj[4];
 #pragma unroll
                 for (int q = 0; q < 4; q++)
-                    if (k0 + q < cnt) pj[q] = ldg_pos(Pj + (ev[q] & NB_INDEX_MASK));
+                    if (left > row_off<TPM>(q)) pj[q] = ldg_pos(Pj + (ev[q] & NB_INDEX_MASK));
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    if (k0 + q >= cnt) break;
+                    if (left <= row_off<TPM>(q)) continue;
                     const int code = ev[q] >> NB_SHIFT_BITS;
                     double xj = pj[q].x, yj = pj[q].y, zj = pj[q].z;
                     if (code != NB_NOSHIFT) {  // rows of boundary cells only

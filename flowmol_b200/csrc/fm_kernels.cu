@@ -16,7 +16,7 @@
 
 #include "fm_common.cuh"
 #include "fm_device.cuh"
-#include "fm_build.cuh"
+#include "fm_force_list.cuh"
 #include "fm_tile.cuh"
 
 namespace fm {
@@ -25,41 +25,6 @@ thread_local bool pdl_capture = false;
 
 namespace {
 
-__device__ __forceinline__ bool frozen(const FmDev &d) { return (d.sc->status & ST_FATAL) != 0u; }
-
-// w of a position: the Mie type (1-based), the Soddemann bead flag (1 for a
-// chain bead), or with both the type plus 32 times the flag.
-__device__ __forceinline__ int mie_type(double w) { return ((int)w) & 31; }
-template <bool MIE>
-__device__ __forceinline__ int bead_flag(double w) { return MIE ? ((int)w) >> 5 : (int)w; }
-
-__device__ __forceinline__ void raise_status(const FmDev &d, uint32_t bit, int iter)
-{
-    if (iter == ITER_DEVICE) iter = d.sc->cur_iter;
-    uint32_t old = atomicOr(&d.sc->status, bit);
-    if ((old & ST_FATAL) == 0u) d.sc->fail_iter = iter;
-}
-
-
-
-
-
-// Block max of a non-negative double folded into sc->vmax2 (u64 order of
-// non-negative doubles equals their numeric order).
-__device__ __forceinline__ void block_vmax2(const FmDev &d, double m2)
-{
-    __shared__ double wmax[32];
-    m2 = warp_max(m2);
-    int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) wmax[w] = m2;
-    __syncthreads();
-    if (w == 0) {
-        int nw = (blockDim.x + 31) >> 5;
-        double v = l < nw ? wmax[l] : 0.0;
-        v = warp_max(v);
-        if (l == 0 && v > 0.0) atomicMax(&d.sc->vmax2, (unsigned long long)__double_as_longlong(v));
-    }
-}
 
 // ---------------------------------------------------------------------------
 // integrator (simulation_move_particles_vv.f90:64-69, 132-135)
@@ -251,12 +216,6 @@ __global__ void k_set_graph_iter(FmDev d, int iter) { d.sc->g_iter = iter; }
 // messenger.serial.f90:961-1028)
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ bool gate(const FmDev &d, int gated)
-{
-    if (frozen(d)) return false;
-    if (gated && !d.sc->rebuild) return false;
-    return true;
-}
 
 
 __global__ void k_wrap_bin(FmDev d, int wrap, int bin, int gated, int iter)
@@ -338,6 +297,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(FmDev d, int gated)
         if (base + k < d.ncell) local += d.cell_count[base + k];
     block_excl_scan(local, &tot);
     if (threadIdx.x == 0) d.tile_sum[blockIdx.x] = tot;
+    if (threadIdx.x == 0 && blockIdx.x == 0) d.sc->strays = 0;  // for k_sort_cells
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(FmDev d, int gated)
@@ -387,34 +347,67 @@ __global__ void k_scatter(FmDev d, int gated)
 // molecules' identity (slot_of: upload index, or global number in a
 // subdomain) makes the whole rebuild deterministic and independent of the
 // previous order, so that a subdomain lays out a cell's molecules exactly as
-// the undivided system does.  One warp per cell: up to 32 members by a
-// bitonic sort of (identity, old slot) keys in registers, larger cells by
-// lane 0 (insertion sort).
+// the undivided system does.  Ahead of the identity goes the octant of the
+// cell (sub_cell), so that the four molecules of a line are near each other
+// and the partners that neighbouring list entries name share lines.  One
+// warp per cell: up to 32 members by a bitonic sort in registers (as many
+// stages as the members need), up to 128 by rank, larger cells by lane 0
+// (insertion sort by identity).
 constexpr int SORT_WARPS = 8;
+constexpr int SORT_RANK = 128;
+__device__ __forceinline__ unsigned long long sort_key(const FmDev &d, const double4 *P, int o, int c)
+{
+    const int ne0 = d.ne[0], ne1 = d.ne[1];
+    const int g0 = c % ne0 + (d.dd ? d.org[0] : 0), g1 = (c / ne0) % ne1 + (d.dd ? d.org[1] : 0);
+    const int g2 = c / (ne0 * ne1) + (d.dd ? d.org[2] : 0);
+    const int oct = sub_cell(P[o], g0, g1, g2, d.hd, d.cs);
+    return (unsigned long long)oct << 32 | (unsigned)d.slot_of[o];
+}
 __global__ void __launch_bounds__(32 * SORT_WARPS) k_sort_cells(FmDev d, int gated)
 {
     pdl_enter();
     if (!gate(d, gated)) return;
     const int lane = threadIdx.x & 31;
+    const double4 *P = cur_pos(d, d.sc->pset);
     for (int c = blockIdx.x * SORT_WARPS + (threadIdx.x >> 5); c < d.ncell; c += gridDim.x * SORT_WARPS) {
         const int b = d.cell_start[c], e = d.cell_start[c + 1];
         const int m = e - b;  // uniform across the warp
         if (m <= 32) {
             unsigned long long key = ~0ull;
+            int o = 0;
             if (lane < m) {
-                const int o = d.perm[b + lane];
-                key = ((unsigned long long)(unsigned)d.slot_of[o] << 32) | (unsigned)o;
+                o = d.perm[b + lane];
+                key = sort_key(d, P, o, c) << 5 | (unsigned)lane;
             }
-#pragma unroll
-            for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
+            for (int k = 2; k < 2 * m; k <<= 1) {
                 for (int j = k >> 1; j > 0; j >>= 1) {
                     const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, j);
                     const bool keep_min = ((lane & j) == 0) == ((lane & k) == 0);
                     key = keep_min ? (key < other ? key : other) : (key > other ? key : other);
                 }
             }
-            if (lane < m) d.perm[b + lane] = (int)(unsigned)(key & 0xffffffffull);
+            o = __shfl_sync(0xffffffffu, o, (int)(key & 31u));
+            if (lane < m) d.perm[b + lane] = o;
+        } else if (m <= SORT_RANK) {
+            unsigned long long key[SORT_RANK / 32];
+            int o[SORT_RANK / 32], rank[SORT_RANK / 32];
+#pragma unroll
+            for (int q = 0; q < SORT_RANK / 32; q++) {
+                const int x = q * 32 + lane;
+                o[q] = x < m ? d.perm[b + x] : 0;
+                key[q] = x < m ? sort_key(d, P, o[q], c) : ~0ull;
+                rank[q] = 0;
+            }
+#pragma unroll
+            for (int p = 0; p < SORT_RANK / 32; p++)
+                for (int l = 0; l < 32; l++) {
+                    const unsigned long long other = __shfl_sync(0xffffffffu, key[p], l);
+#pragma unroll
+                    for (int q = 0; q < SORT_RANK / 32; q++) rank[q] += other < key[q] ? 1 : 0;
+                }
+#pragma unroll
+            for (int q = 0; q < SORT_RANK / 32; q++)
+                if (q * 32 + lane < m) d.perm[b + rank[q]] = o[q];
         } else if (lane == 0) {
             for (int x = b + 1; x < e; x++) {
                 const int o = d.perm[x];
@@ -427,7 +420,14 @@ __global__ void __launch_bounds__(32 * SORT_WARPS) k_sort_cells(FmDev d, int gat
                 d.perm[y + 1] = o;
             }
         }
-        if (lane == 0) d.cell_count[c] = 0;  // leave counts zeroed for the next histogram
+        for (int k = b + lane; k < e; k += 32) d.cell_of[k] = c;  // by new slot from here on
+        if (lane == 0) {
+            d.cell_count[c] = 0;  // leave counts zeroed for the next histogram
+            if (m > 0 && !d.dd) {
+                const int cx = c % d.ne[0], cy = (c / d.ne[0]) % d.ne[1], cz = c / (d.ne[0] * d.ne[1]);
+                if (is_halo(cx, d.ne[0]) || is_halo(cy, d.ne[1]) || is_halo(cz, d.ne[2])) d.sc->strays = 1;
+            }
+        }
     }
 }
 
@@ -514,416 +514,10 @@ __global__ void __launch_bounds__(BS_THREADS) k_blk_seg(FmDev d, int gated, int 
     }
 }
 
-// Neighbour rows of every extended cell, one warp per cell or, for sparse
-// systems (BLOCKS), per block of 2x2x2 cells (grid-stride); the routines and
-// their pair-set argument are in fm_build.cuh.  Both give the same rows.
-template <bool POLY, bool BLOCKS, bool TILE>
-__global__ void __launch_bounds__(NB_THREADS, 8) k_build_nlist(FmDev d, int gated, int iter)
-{
-    pdl_enter();
-    if (!gate(d, gated)) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    using Shared = typename std::conditional<BLOCKS, BlockShared<POLY, TILE>, BuildShared<POLY, TILE>>::type;
-    // per-warp staging in dynamic shared memory (the largest variants pass 48 KB)
-    extern __shared__ __align__(16) unsigned char build_smem[];
-    Shared *sh = reinterpret_cast<Shared *>(build_smem);
-    CellSys y;
-    y.P = cur_pos(d, d.sc->pset);
-    y.cell_start = d.cell_start;
-    y.mol_off = 0;
-    for (int k = 0; k < 3; k++) { y.ne[k] = d.ne[k]; y.cs[k] = d.cs[k]; y.hd[k] = d.hd[k]; y.L[k] = d.L[k]; }
-    y.rn2 = d.rn2;
-    y.nbr = d.nbr;
-    y.nnbr = d.nnbr;
-    y.maxn = d.maxn;
-    y.max_nbr = &d.sc->max_nbr;
-    y.chain = d.chain; y.subchain = d.subchain; y.bflag = d.bflag;
-    y.bnd = d.bnd; y.nbond = d.nbond;
-    y.nbr16 = d.nbr16; y.maxn16 = d.maxn16; y.tT = d.tile_T; y.tR = d.tile_R; y.blk_off = d.blk_off;
-    y.tdummy = d.tile ? tile_boff(d.tile_ucap, d.tile_R) : 0;
-    for (int k = 0; k < 3; k++) y.tnb[k] = d.tile_nb[k];
-    y.dd = d.dd;
-    for (int k = 0; k < 3; k++) y.org[k] = d.dd ? d.org[k] : 0;
-    uint32_t over = 0u;
-    const int nwork = BLOCKS ? ((d.ne[0] + 1) / 2) * ((d.ne[1] + 1) / 2) * ((d.ne[2] + 1) / 2) : d.ncell;
-    // work units handed out NB_CHUNK at a time, so warps that meet empty or
-    // halo cells take more: no tail of a few warps with dense cells left
-    for (;;) {
-        int u0 = 0;
-        if (lane == 0) u0 = atomicAdd(&d.sc->build_next, NB_CHUNK);
-        u0 = __shfl_sync(0xffffffffu, u0, 0);
-        if (u0 >= nwork) break;
-        const int u1 = min(u0 + NB_CHUNK, nwork);
-        for (int u = u0; u < u1; u++) {
-            if constexpr (BLOCKS) over |= build_block<POLY, TILE>(y, u, sh[warp], lane);
-            else over |= build_cell<POLY, TILE>(y, u, sh[warp], lane);
-        }
-    }
-    if (lane == 0) {
-        if (over & BUILD_OVER_LIST) raise_status(d, ST_NLIST, iter);
-        if (over & BUILD_OVER_BONDS) raise_status(d, ST_BOND, iter);
-    }
-}
-
 // ---------------------------------------------------------------------------
 // forces (simulation_compute_forces_LJ_neigbr*, simulation_compute_forces.f90
 // :551-726) fused with move(2) and the next move(1)
 // ---------------------------------------------------------------------------
-
-constexpr int FORCE_THREADS = 256;
-
-// One pair inside the cutoff: acc (the pair force over rij) accumulated as
-// acc * rij, and on record steps the energy and acc * r^2.  PREC bit 0: FP32
-// pair magnitude (FP64 rij scales it); bit 1: Mie_potential 1, constants by
-// the molecules' types (w of the positions): Mie_accijmag and Mie_energy
-// (setup_set_parameters.f90:149-204) with real powers, as s**(lr/2+1).
-// Otherwise LJ_accijmag = 48 (s^7 - s^4/2), s = 1/r^2, and LJ_energy
-// (:105-135).
-template <int PREC, bool REC>
-__device__ __forceinline__ double pair_acc(const FmDev &d, double r2, double dx, double dy, double dz, double wi,
-                                           double wj, double &fx, double &fy, double &fz, double &pe, double &vir)
-{
-    constexpr bool F32 = (PREC & 1) != 0, MIE = (PREC & 2) != 0, SOD = (PREC & 4) != 0;
-    if (SOD) {
-        // simulation_compute_forces_Soddemann_neigbr_halfint (:793-888): WCA
-        // inside wca_cut2, the cosine well eps a s^2 sin(a s + b) beyond it
-        // (the reference's expression, s = 1/r^2); no potshift.  The WCA force
-        // is get_accijmag: Mie_accijmag of the pair's types with
-        // Mie_potential 1, its energy the LJ-WCA expression either way.
-        const double eps = d.sod_eps[bead_flag<MIE>(wi) + bead_flag<MIE>(wj)];
-        const bool wca = r2 < SOD_WCA_CUT2;
-        if (!F32) {
-            const double s = __drcp_rn(r2);
-            const double s2 = s * s;
-            double acc;
-            if (wca && MIE) {
-                const FmMiePair &m = d.mie_pair[(mie_type(wi) - 1) + MIE_MAXT * (mie_type(wj) - 1)];
-                acc = m.ceps * (m.lr * pow(s, m.er1) - m.ala * pow(s, m.ea1));
-            } else if (wca) {
-                const double s4 = s2 * s2;
-                acc = 48.0 * (s4 * s2 * s - 0.5 * s4);  // get_accijmag = LJ_accijmag
-            } else {
-                acc = (eps * SOD_A * s2) * sin(s * SOD_A + SOD_B);
-            }
-            fx += acc * dx; fy += acc * dy; fz += acc * dz;
-            if (REC) {
-                if (wca) {
-                    const double s3 = s2 * s, s6 = s3 * s3;
-                    pe += 4.0 * (s6 - s3 + 0.25) - eps;
-                } else {
-                    pe += 0.5 * eps * (cos(SOD_A * r2 + SOD_B) - 1.0);
-                }
-                vir += acc * r2;
-            }
-        } else {
-            const float s = rcp_f32((float)r2);
-            const float s2 = s * s;
-            float accf;
-            if (wca && MIE) {
-                const FmMiePair &m = d.mie_pair[(mie_type(wi) - 1) + MIE_MAXT * (mie_type(wj) - 1)];
-                accf = (float)m.ceps * ((float)m.lr * powf(s, (float)m.er1) - (float)m.ala * powf(s, (float)m.ea1));
-            } else if (wca) {
-                const float s4 = s2 * s2;
-                accf = 48.0f * (s4 * s2 * s - 0.5f * s4);
-            } else {
-                accf = ((float)eps * (float)SOD_A * s2) * sinf(s * (float)SOD_A + (float)SOD_B);
-            }
-            const double acc = (double)accf;
-            fx = fma(acc, dx, fx); fy = fma(acc, dy, fy); fz = fma(acc, dz, fz);
-            if (REC) {
-                if (wca) {
-                    const float s3 = s2 * s, s6 = s3 * s3;
-                    pe += (double)(4.0f * (s6 - s3 + 0.25f)) - eps;
-                } else {
-                    pe += (double)(0.5f * (float)eps * (cosf((float)SOD_A * (float)r2 + (float)SOD_B) - 1.0f));
-                }
-                vir += acc * r2;
-            }
-        }
-        return 0.0;  // the Soddemann routine records no pressure-tensor term
-    }
-    if (MIE) {
-        const FmMiePair &m = d.mie_pair[(mie_type(wi) - 1) + MIE_MAXT * (mie_type(wj) - 1)];
-        if (!F32) {
-            const double s = __drcp_rn(r2);  // == 1.0 / r2
-            const double acc = m.ceps * (m.lr * pow(s, m.er1) - m.ala * pow(s, m.ea1));
-            fx += acc * dx; fy += acc * dy; fz += acc * dz;
-            if (REC) {
-                pe += m.ceps * (pow(s, m.er) - m.alpha * pow(s, m.ea)) - m.shift;
-                vir += acc * r2;
-            }
-            return acc;
-        } else {
-            const float s = rcp_f32((float)r2);
-            const double acc = (double)((float)m.ceps * ((float)m.lr * powf(s, (float)m.er1) -
-                                                         (float)m.ala * powf(s, (float)m.ea1)));
-            fx = fma(acc, dx, fx); fy = fma(acc, dy, fy); fz = fma(acc, dz, fz);
-            if (REC) {
-                pe += (double)((float)m.ceps * (powf(s, (float)m.er) - (float)m.alpha * powf(s, (float)m.ea))) - m.shift;
-                vir += acc * r2;
-            }
-            return acc;
-        }
-    } else if (!F32) {
-        const double s = __drcp_rn(r2);  // == 1.0 / r2 (both correctly rounded)
-        const double s2 = s * s, s4 = s2 * s2;
-        const double acc = 48.0 * (s4 * s2 * s - 0.5 * s4);
-        fx += acc * dx; fy += acc * dy; fz += acc * dz;
-        if (REC) {
-            const double s3 = s2 * s, s6 = s3 * s3;
-            pe += 4.0 * (s6 - s3) - d.potshift;  // LJ_energy (:126-135)
-            vir += acc * r2;
-        }
-        return acc;
-    } else {
-        // FP32 pair magnitude; the FP64 rij scales it (one conversion)
-        const float s = rcp_f32((float)r2);
-        const float s2 = s * s, s4 = s2 * s2;
-        const double acc = (double)(48.0f * (s4 * s2 * s - 0.5f * s4));
-        fx = fma(acc, dx, fx); fy = fma(acc, dy, fy); fz = fma(acc, dz, fz);
-        if (REC) {
-            const float s3 = s2 * s, s6 = s3 * s3;
-            pe += (double)(4.0f * (s6 - s3)) - d.potshift;
-            vir += acc * r2;
-        }
-        return acc;
-    }
-}
-
-// pressure_tensor_forces (simulation_record.f90:6239-6256): rf += acc rij rij,
-// the six distinct components xx yy zz xy xz yz.
-__device__ __forceinline__ void add_rf(double (&rf)[6], double acc, double dx, double dy, double dz)
-{
-    const double ax = acc * dx, ay = acc * dy, az = acc * dz;
-    rf[0] += ax * dx; rf[1] += ay * dy; rf[2] += az * dz;
-    rf[3] += ax * dy; rf[4] += ax * dz; rf[5] += ay * dz;
-}
-
-// Record-step pressure terms of one molecule: v v + rf/2 (cumulative_pressure
-// case 1, simulation_record.f90:3170-3199; no mass factor there).
-__device__ __forceinline__ void pressure_part(double (&part)[RS_N], double wx, double wy, double wz,
-                                              const double (&rf)[6])
-{
-    part[RS_PXX] = wx * wx + rf[0] / 2.0; part[RS_PYY] = wy * wy + rf[1] / 2.0;
-    part[RS_PZZ] = wz * wz + rf[2] / 2.0; part[RS_PXY] = wx * wy + rf[3] / 2.0;
-    part[RS_PXZ] = wx * wz + rf[4] / 2.0; part[RS_PYZ] = wy * wz + rf[5] / 2.0;
-}
-
-// Integrator epilogue of molecule i with its summed LJ force: stores a (and PE
-// and virial on record steps) and, by MODE,
-//   1  move(2)                               (simulation_move_particles_vv.f90:132-135)
-//   2  move(2) + move(1) of the next step    (:64-69), new positions into pset^1
-//   3  leap-frog v += dt a, r += dt v        (simulation_move_particles_lfv.f90:81-92)
-// The record partials use v after move(2) for velocity Verlet and v + a dt/2
-// for leap-frog (simulation_record.f90:1236-1252).  Returns |v|^2 after a
-// position update (modes 2, 3), else 0.
-// DIV false: the forces are accelerations already (the Soddemann pairs and
-// the mass-divided bonds of a Mie + Soddemann system); the kinetic terms are
-// still mass-weighted.
-template <bool REC, int MODE, bool MIE = false, bool DIV = true>
-__device__ __forceinline__ double epilogue(const FmDev &d, int pset, int i, double4 p, double fx, double fy,
-                                           double fz, double pe, double vir, double (&part)[RS_N],
-                                           const double (&rf)[6])
-{
-    if (REC && d.pressure) {  // kept for a record taken after the move (fm_evaluate_macroscopic_properties)
-        double *q = d.rf6 + 6 * (size_t)i;
-#pragma unroll
-        for (int k = 0; k < 6; k++) q[k] = rf[k];
-    }
-    double mass = 1.0;  // LJ_mass; Mie_mass = mass_lookup(moltype)
-    if (MIE) {
-        mass = d.mie_mass[mie_type(p.w) - 1];
-        if (DIV) { fx = fx / mass; fy = fy / mass; fz = fz / mass; }
-    }
-    d.ax[i] = fx; d.ay[i] = fy; d.az[i] = fz;
-    if (REC) { d.pe[i] = pe; d.vir[i] = vir; }
-    double vx = d.vx[i], vy = d.vy[i], vz = d.vz[i];
-    double m2 = 0.0;
-    if (MODE == 3) {
-        if (REC) {
-            const double wx = __dadd_rn(vx, __dmul_rn(__dmul_rn(0.5, fx), d.dt));
-            const double wy = __dadd_rn(vy, __dmul_rn(__dmul_rn(0.5, fy), d.dt));
-            const double wz = __dadd_rn(vz, __dmul_rn(__dmul_rn(0.5, fz), d.dt));
-            part[RS_PE] = pe; part[RS_VIR] = vir; part[RS_PEMAX] = pe;
-            part[RS_MV2] = MIE ? mass * norm2_rn(wx, wy, wz) : norm2_rn(wx, wy, wz);
-            part[RS_VSUM] = MIE ? mass * __dadd_rn(__dadd_rn(wx, wy), wz) : __dadd_rn(__dadd_rn(wx, wy), wz);
-            if (d.pressure) pressure_part(part, wx, wy, wz, rf);
-        }
-        vx = __dadd_rn(vx, __dmul_rn(d.dt, fx));
-        vy = __dadd_rn(vy, __dmul_rn(d.dt, fy));
-        vz = __dadd_rn(vz, __dmul_rn(d.dt, fz));
-        p.x = __dadd_rn(p.x, __dmul_rn(d.dt, vx));
-        p.y = __dadd_rn(p.y, __dmul_rn(d.dt, vy));
-        p.z = __dadd_rn(p.z, __dmul_rn(d.dt, vz));
-        cur_pos(d, pset ^ 1)[i] = p;
-        d.vx[i] = vx; d.vy[i] = vy; d.vz[i] = vz;
-        return norm2_rn(vx, vy, vz);
-    }
-    if (MODE >= 1) {
-        vx = __dadd_rn(vx, __dmul_rn(d.half_dt, fx));
-        vy = __dadd_rn(vy, __dmul_rn(d.half_dt, fy));
-        vz = __dadd_rn(vz, __dmul_rn(d.half_dt, fz));
-    }
-    if (REC) {
-        double wx = vx, wy = vy, wz = vz;
-        if (MODE == 0 && d.integrator == 0) {  // forces only, leap-frog record velocity
-            wx = __dadd_rn(vx, __dmul_rn(__dmul_rn(0.5, fx), d.dt));
-            wy = __dadd_rn(vy, __dmul_rn(__dmul_rn(0.5, fy), d.dt));
-            wz = __dadd_rn(vz, __dmul_rn(__dmul_rn(0.5, fz), d.dt));
-        }
-        part[RS_PE] = pe; part[RS_VIR] = vir; part[RS_PEMAX] = pe;
-        part[RS_MV2] = MIE ? mass * norm2_rn(wx, wy, wz) : norm2_rn(wx, wy, wz);
-        part[RS_VSUM] = MIE ? mass * __dadd_rn(__dadd_rn(wx, wy), wz) : __dadd_rn(__dadd_rn(wx, wy), wz);
-        if (d.pressure) pressure_part(part, wx, wy, wz, rf);
-    }
-    if (MODE == 2) {
-        p.x = __dadd_rn(__dadd_rn(p.x, __dmul_rn(d.dt, vx)), __dmul_rn(d.half_dt2, fx));
-        p.y = __dadd_rn(__dadd_rn(p.y, __dmul_rn(d.dt, vy)), __dmul_rn(d.half_dt2, fy));
-        p.z = __dadd_rn(__dadd_rn(p.z, __dmul_rn(d.dt, vz)), __dmul_rn(d.half_dt2, fz));
-        vx = __dadd_rn(vx, __dmul_rn(d.half_dt, fx));
-        vy = __dadd_rn(vy, __dmul_rn(d.half_dt, fy));
-        vz = __dadd_rn(vz, __dmul_rn(d.half_dt, fz));
-        cur_pos(d, pset ^ 1)[i] = p;
-        m2 = norm2_rn(vx, vy, vz);
-    }
-    if (MODE >= 1) { d.vx[i] = vx; d.vy[i] = vy; d.vz[i] = vz; }
-    return m2;
-}
-
-// FENE springs of molecule i (simulation_compute_forces_poly,
-// simulation_compute_forces.f90:731-789): accijmag = -k/(1 - r^2/R0^2)
-// (FENE_accijmag, setup_set_parameters.f90:348-358), energy
-// 0.5 k R0^2 log(1 - r^2/R0^2) (:371-380), in FP64 for every precision form.
-// A bond at or beyond R0 is the reference's polymer_bond_error.
-template <bool REC, bool MIE>
-__device__ __forceinline__ void fene_bonds(const FmDev &d, const double4 *P, int i, double &fx, double &fy,
-                                           double &fz, double &pe, double &vir, double (&rf)[6])
-{
-    const double4 pi = P[i];
-    const int nb = d.nbond[i];
-    for (int b = 0; b < nb; b++) {
-        const int e = d.bnd[(size_t)i * 4 + b];
-        const int code = e >> NB_SHIFT_BITS;
-        const double4 pj = P[e & NB_INDEX_MASK];
-        const double xj = (code & 3) != 1 ? __dadd_rn(pj.x, (code & 3) == 2 ? d.L[0] : -d.L[0]) : pj.x;
-        const double yj = ((code >> 2) & 3) != 1 ? __dadd_rn(pj.y, ((code >> 2) & 3) == 2 ? d.L[1] : -d.L[1]) : pj.y;
-        const double zj = ((code >> 4) & 3) != 1 ? __dadd_rn(pj.z, ((code >> 4) & 3) == 2 ? d.L[2] : -d.L[2]) : pj.z;
-        const double dx = __dsub_rn(pi.x, xj), dy = __dsub_rn(pi.y, yj), dz = __dsub_rn(pi.z, zj);
-        const double r2 = norm2_rn(dx, dy, dz);
-        if (MIE) {
-            // harmonic_accijmag / harmonic_energy (setup_set_parameters.f90:384-437):
-            // -k (|r| - r0)/|r| and k/2 (|r| - r0)^2, constants by type pair
-            const FmMiePair &m = d.mie_pair[(mie_type(pi.w) - 1) + MIE_MAXT * (mie_type(pj.w) - 1)];
-            const double rm = sqrt(r2), dr = rm - m.r0;
-            const double acc = -m.k * dr / rm;
-            fx += acc * dx; fy += acc * dy; fz += acc * dz;
-            if (REC) {
-                pe += 0.5 * m.k * (dr * dr);
-                vir += acc * r2;
-                if (d.pressure) add_rf(rf, acc, dx, dy, dz);  // :768-770
-            }
-            continue;
-        }
-        if (r2 >= d.R0_2) {
-            uint32_t old = atomicOr(&d.sc->status, ST_BOND);
-            if ((old & ST_FATAL) == 0u) d.sc->fail_iter = -2;
-            continue;
-        }
-        const double q = r2 / d.R0_2;
-        const double acc = -d.k_c / (1.0 - q);
-        fx += acc * dx; fy += acc * dy; fz += acc * dz;
-        if (REC) {
-            pe += 0.5 * d.k_c * d.R0 * d.R0 * log(1.0 - q);
-            vir += acc * r2;
-            if (d.pressure) add_rf(rf, acc, dx, dy, dz);  // :768-770
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// angular_potential (simulation_compute_forces_angular,
-// simulation_compute_forces.f90:981-1048; angular_harmonic_force,
-// setup_set_parameters.f90:441-489)
-// ---------------------------------------------------------------------------
-
-// The reference's triple of middle bead j: i = its first bond, k = its second
-// (in discovery order), rij = r_i - r_j, rjk = r_j - r_k with the partners'
-// periodic images (x_src +/- L, one rounding), theta = acos(rij.rjk /
-// (|rij| |rjk|)) and
-//   aForce(1) = -(k (theta - theta_0) / (|rij| sin theta)) (rjk/|rjk| - rij/|rij| cos theta)
-//   aForce(3) = -(k (theta - theta_0) / (|rjk| sin theta)) (rij/|rij| - rjk/|rjk| cos theta)
-//   aForce(2) = -aForce(1) - aForce(3)   (all zero when theta < 1e-5);
-// the reference then subtracts aForce(1), (2), (3) from the forces on i, j,
-// k.  Every molecule evaluates the triples it belongs to in the middle
-// bead's frame, so the three see the same numbers.  k_ijk < 1e-5 leaves the
-// reference's result unset: ST_ANGLE.
-__device__ __forceinline__ bool angular_triple(const FmDev &d, const double4 *P, int j, double (&f1)[3],
-                                               double (&f3)[3])
-{
-    const int e0 = d.bnd[(size_t)j * 4], e1 = d.bnd[(size_t)j * 4 + 1];
-    const double4 pj = P[j], pi = P[e0 & NB_INDEX_MASK], pk = P[e1 & NB_INDEX_MASK];
-    const int c0 = e0 >> NB_SHIFT_BITS, c1 = e1 >> NB_SHIFT_BITS;
-    const double ri[3] = {image(pi.x, (c0 & 3) - 1, d.L[0]), image(pi.y, ((c0 >> 2) & 3) - 1, d.L[1]),
-                          image(pi.z, ((c0 >> 4) & 3) - 1, d.L[2])};
-    const double rk[3] = {image(pk.x, (c1 & 3) - 1, d.L[0]), image(pk.y, ((c1 >> 2) & 3) - 1, d.L[1]),
-                          image(pk.z, ((c1 >> 4) & 3) - 1, d.L[2])};
-    const double rj[3] = {pj.x, pj.y, pj.z};
-    const int nt = d.ang_nt;
-    const int q = (mie_type(pi.w) - 1) + nt * ((mie_type(pj.w) - 1) + nt * (mie_type(pk.w) - 1));
-    const double kk = d.ang_k[q], t0 = d.ang_t0[q];
-    f1[0] = f1[1] = f1[2] = 0.0;
-    f3[0] = f3[1] = f3[2] = 0.0;
-    if (kk < 1e-5) return false;
-    double rij[3], rjk[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) { rij[c] = __dsub_rn(ri[c], rj[c]); rjk[c] = __dsub_rn(rj[c], rk[c]); }
-    const double mij = sqrt(norm2_rn(rij[0], rij[1], rij[2]));
-    const double mjk = sqrt(norm2_rn(rjk[0], rjk[1], rjk[2]));
-    const double dot = __dadd_rn(__dadd_rn(__dmul_rn(rij[0], rjk[0]), __dmul_rn(rij[1], rjk[1])),
-                                 __dmul_rn(rij[2], rjk[2]));
-    const double th = acos(dot / (mij * mjk));
-    if (th < 1e-5) return true;
-    const double ct = cos(th), stt = sin(th);
-    const double a1 = kk * (th - t0) / (mij * stt), a3 = kk * (th - t0) / (mjk * stt);
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        f1[c] = -a1 * (rjk[c] / mjk - rij[c] / mij * ct);
-        f3[c] = -a3 * (rij[c] / mij - rjk[c] / mjk * ct);
-    }
-    return true;
-}
-
-// The angular forces on molecule m (added to its force sum before the
-// division by its mass): -aForce(2) of its own triple when it is a middle
-// bead, and -aForce(1) or -aForce(3) of each bonded middle bead's triple in
-// which it is the bead i or k.
-__device__ __forceinline__ void angular_forces(const FmDev &d, const double4 *P, int m, double &fx, double &fy,
-                                               double &fz)
-{
-    double f1[3], f3[3];
-    bool ok = true;
-    if (d.funcy[m] == 2) {
-        ok &= angular_triple(d, P, m, f1, f3);
-        fx += f1[0] + f3[0]; fy += f1[1] + f3[1]; fz += f1[2] + f3[2];  // -aForce(2)
-    }
-    const int nb = d.nbond[m];
-    for (int b = 0; b < nb; b++) {
-        const int e = d.bnd[(size_t)m * 4 + b];
-        const int p = e & NB_INDEX_MASK;
-        if (d.funcy[p] != 2) continue;
-        const int c = e >> NB_SHIFT_BITS;  // m as p sees it: the opposite image
-        const int back = m | (((2 - (c & 3)) | ((2 - ((c >> 2) & 3)) << 2) | ((2 - ((c >> 4) & 3)) << 4))
-                              << NB_SHIFT_BITS);
-        ok &= angular_triple(d, P, p, f1, f3);
-        if (d.bnd[(size_t)p * 4] == back) { fx -= f1[0]; fy -= f1[1]; fz -= f1[2]; }
-        else if (d.bnd[(size_t)p * 4 + 1] == back) { fx -= f3[0]; fy -= f3[1]; fz -= f3[2]; }
-        else ok = false;
-    }
-    if (!ok) {
-        uint32_t old = atomicOr(&d.sc->status, ST_ANGLE);
-        if ((old & ST_FATAL) == 0u) d.sc->fail_iter = -3;
-    }
-}
 
 // Discovery key of the bond (j, entry) in the reference's list build
 // (assign_to_neighbourlist_halfint_opt, linklist.f90:660-804, where
@@ -996,158 +590,6 @@ __global__ void k_set_funcy(FmDev d, const int32_t *funcy_up)
 {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u < d.n) d.funcy[u] = funcy_up[u];  // slots still equal upload indices
-}
-
-// (s, c) += (s2, c2): Neumaier merge of two compensated partial sums.
-__device__ __forceinline__ void nmerge(double &s, double &c, double s2, double c2)
-{
-    neumaier(s, c, s2);
-    c += c2;
-}
-
-// Block reduction of the record partials into row `row` of d.partial:
-// Neumaier-compensated sums in a fixed tree order (warp xor tree, then the
-// warps in index order), the row holding the compensated value rounded once;
-// PE max for the PE check.
-template <int NT = FORCE_THREADS>
-__device__ __forceinline__ void block_partials(const FmDev &d, double v[RS_N], int row)
-{
-    __shared__ double ws[RS_N][NT / 32], wc[RS_N][NT / 32];
-    int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const int nq = d.pressure ? (int)RS_N : (int)RS_PXX;  // the pressure terms only where they are summed
-#pragma unroll
-    for (int k = 0; k < RS_N; k++) {
-        if (k >= nq) break;
-        double x = v[k], c = 0.0;
-        if (k == RS_PEMAX) {
-            x = warp_max(x);
-        } else {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double x2 = __shfl_xor_sync(0xffffffffu, x, o), c2 = __shfl_xor_sync(0xffffffffu, c, o);
-                nmerge(x, c, x2, c2);
-            }
-        }
-        if (l == 0) { ws[k][w] = x; wc[k][w] = c; }
-    }
-    __syncthreads();
-    if (threadIdx.x < nq) {
-        int k = threadIdx.x;
-        double acc = ws[k][0], cmp = wc[k][0];
-        for (int q = 1; q < NT / 32; q++) {
-            if (k == RS_PEMAX) acc = fmax(acc, ws[k][q]);
-            else nmerge(acc, cmp, ws[k][q], wc[k][q]);
-        }
-        d.partial[(size_t)row * RS_N + k] = k == RS_PEMAX ? acc : acc + cmp;
-    }
-}
-
-// Pair sum of molecule i over its list row: lane `lane` of the molecule's
-// TPM lanes takes 4 consecutive entries per iteration (one 16-byte load) and
-// issues their 4 gathers before any arithmetic.  Entries without an image
-// shift (all but the rows of boundary cells) skip the shift decoding.
-template <int TPM, bool REC, int PREC>
-__device__ __forceinline__ void list_pairs(const FmDev &d, const double4 *__restrict__ P, int i, int lane,
-                                           const double4 &pi, double &fx, double &fy, double &fz, double &pe,
-                                           double &vir, double (&rf)[6])
-{
-    const int cnt = d.nnbr[i];
-    const int32_t *__restrict__ L = d.nbr + nb_row(i, d.maxn);  // entries k0..k0+3 at L + nb_col(k0) (16-byte aligned)
-    const double Lx = d.L[0], Ly = d.L[1], Lz = d.L[2];
-    const double rc2 = d.rc2;
-    for (int k0 = lane * 4; k0 < cnt; k0 += 4 * TPM) {
-        const int4 e4 = ld_stream_int4(reinterpret_cast<const int4 *>(L + nb_col(k0)));
-        const int ev[4] = {e4.x, e4.y, e4.z, e4.w};
-        double4 pj[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-            if (k0 + q < cnt) pj[q] = ldg_pos(P + (ev[q] & NB_INDEX_MASK));
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            if (k0 + q >= cnt) break;
-            const int code = ev[q] >> NB_SHIFT_BITS;
-            double xj = pj[q].x, yj = pj[q].y, zj = pj[q].z;
-            if (code != NB_NOSHIFT) {
-                const int ssx = (code & 3) - 1, ssy = ((code >> 2) & 3) - 1, ssz = ((code >> 4) & 3) - 1;
-                xj = ssx ? __dadd_rn(xj, ssx > 0 ? Lx : -Lx) : xj;
-                yj = ssy ? __dadd_rn(yj, ssy > 0 ? Ly : -Ly) : yj;
-                zj = ssz ? __dadd_rn(zj, ssz > 0 ? Lz : -Lz) : zj;
-            }
-            const double dx = __dsub_rn(pi.x, xj);
-            const double dy = __dsub_rn(pi.y, yj);
-            const double dz = __dsub_rn(pi.z, zj);
-            const double r2 = norm2_rn(dx, dy, dz);
-            if (r2 < rc2) {
-                const double acc = pair_acc<PREC, REC>(d, r2, dx, dy, dz, pi.w, pj[q].w, fx, fy, fz, pe, vir);
-                // every partner of i in the full list: the half list's i and j sides
-                if (REC && d.pressure) add_rf(rf, acc, dx, dy, dz);
-            }
-        }
-    }
-}
-
-// Bonded terms and the integrator epilogue of molecule i once its pair sum is
-// complete; returns |v|^2 after a position update (epilogue()).
-template <bool REC, int MODE, int PREC>
-__device__ __forceinline__ double owner_finish(const FmDev &d, int pset, const double4 *__restrict__ P, int i,
-                                               double fx, double fy, double fz, double pe, double vir,
-                                               double (&part)[RS_N], double (&rf)[6])
-{
-    if constexpr ((PREC & 6) == 6) {
-        // Mie + Soddemann: the Soddemann pairs are not divided by a mass
-        // (:852-860), the bonds of simulation_compute_forces_poly are
-        // (:752-754)
-        const double4 pi = P[i];
-        double bx = 0.0, by = 0.0, bz = 0.0;
-        if (d.potential_flag == 1) fene_bonds<REC, true>(d, P, i, bx, by, bz, pe, vir, rf);
-        const double mass = d.mie_mass[mie_type(pi.w) - 1];
-        fx += bx / mass; fy += by / mass; fz += bz / mass;
-        return epilogue<REC, MODE, true, false>(d, pset, i, pi, fx, fy, fz, pe, vir, part, rf);
-    } else {
-        if (d.potential_flag == 1) fene_bonds<REC, (PREC & 2) != 0>(d, P, i, fx, fy, fz, pe, vir, rf);
-        if constexpr ((PREC & 2) != 0) {  // angular_potential needs the Mie types
-            if (d.angular) angular_forces(d, P, i, fx, fy, fz);
-        }
-        // a(:,i) = sum acc rij / mass (LJ_mass = 1; Mie_mass by type)
-        return epilogue<REC, MODE, (PREC & 2) != 0>(d, pset, i, P[i], fx, fy, fz, pe, vir, part, rf);
-    }
-}
-
-template <int TPM, bool REC, int MODE, int PREC>
-__global__ void __launch_bounds__(FORCE_THREADS) k_force(FmDev d)
-{
-    pdl_enter();
-    if (frozen(d)) return;
-    const int pset = d.sc->pset;
-    const double4 *__restrict__ P = cur_pos(d, pset);
-    const int gt = blockIdx.x * FORCE_THREADS + threadIdx.x;
-    const int i = gt / TPM;
-    const int lane = gt % TPM;
-    const bool active = i < d.n;
-    double fx = 0.0, fy = 0.0, fz = 0.0, pe = 0.0, vir = 0.0;
-    double rf[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    if (active) list_pairs<TPM, REC, PREC>(d, P, i, lane, P[i], fx, fy, fz, pe, vir, rf);
-    if (TPM > 1) {
-#pragma unroll
-        for (int o = TPM / 2; o > 0; o >>= 1) {
-            fx += __shfl_xor_sync(0xffffffffu, fx, o);
-            fy += __shfl_xor_sync(0xffffffffu, fy, o);
-            fz += __shfl_xor_sync(0xffffffffu, fz, o);
-            if (REC) {
-                pe += __shfl_xor_sync(0xffffffffu, pe, o);
-                vir += __shfl_xor_sync(0xffffffffu, vir, o);
-                if (d.pressure) {
-#pragma unroll
-                    for (int k = 0; k < 6; k++) rf[k] += __shfl_xor_sync(0xffffffffu, rf[k], o);
-                }
-            }
-        }
-    }
-    double part[RS_N] = {};
-    double m2 = 0.0;
-    if (active && lane == 0) m2 = owner_finish<REC, MODE, PREC>(d, pset, P, i, fx, fy, fz, pe, vir, part, rf);
-    if (REC) block_partials(d, part, blockIdx.x);
-    if (MODE >= 2) block_vmax2(d, m2);
 }
 
 // ---------------------------------------------------------------------------
@@ -1731,57 +1173,6 @@ void launch_reorder(const FmDev &d, int gated, double4 *tpos, int32_t *tuidx, cu
     pdl_launch(k_reorder_gather, sgrid(d.n, 256, 8), 256, st, d, gated, tpos, tuidx);
     pdl_launch(k_reorder_copy, sgrid(d.n, 256, 8), 256, st, d, gated, tpos, tuidx);
 }
-// The list build walks the cells grid-stride with every block resident (one
-// wave: a second partial wave would double the kernel's time).
-template <bool POLY, bool BLOCKS, bool TILE>
-static size_t build_smem_bytes()
-{
-    using Shared = typename std::conditional<BLOCKS, BlockShared<POLY, TILE>, BuildShared<POLY, TILE>>::type;
-    return sizeof(Shared) * NB_WARPS;
-}
-
-template <bool POLY, bool BLOCKS, bool TILE>
-static int build_grid(int nwork)
-{
-    static int resident = 0;
-    if (resident == 0) {
-        int dev = 0, nsm = kSMs, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(k_build_nlist<POLY, BLOCKS, TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)build_smem_bytes<POLY, BLOCKS, TILE>());
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_build_nlist<POLY, BLOCKS, TILE>, NB_THREADS,
-                                                      build_smem_bytes<POLY, BLOCKS, TILE>());
-        resident = std::max(nsm, 1) * std::max(per_sm, 1);
-    }
-    return std::min(nblk(nwork, NB_WARPS), resident);
-}
-
-template <bool POLY, bool BLOCKS, bool TILE>
-static void launch_build_t(const FmDev &d, int nwork, int gated, int iter, cudaStream_t st)
-{
-    const int g = build_grid<POLY, BLOCKS, TILE>(nwork);  // (sets the kernel's shared-memory attribute once)
-    pdl_launch_smem(k_build_nlist<POLY, BLOCKS, TILE>, g, NB_THREADS, build_smem_bytes<POLY, BLOCKS, TILE>(), st, d,
-                    gated, iter);
-}
-
-void launch_build_nlist(const FmDev &d, int gated, int iter, cudaStream_t st)
-{
-    cudaMemsetAsync(&d.sc->build_next, 0, sizeof(int32_t), st);
-    const int nb = ((d.ne[0] + 1) / 2) * ((d.ne[1] + 1) / 2) * ((d.ne[2] + 1) / 2);
-    const int nw = d.build_blocks ? nb : d.ncell;
-    switch ((d.potential_flag == 1 ? 4 : 0) + (d.build_blocks ? 2 : 0) + (d.tile ? 1 : 0)) {
-    case 0: launch_build_t<false, false, false>(d, nw, gated, iter, st); break;
-    case 1: launch_build_t<false, false, true>(d, nw, gated, iter, st); break;
-    case 2: launch_build_t<false, true, false>(d, nw, gated, iter, st); break;
-    case 3: launch_build_t<false, true, true>(d, nw, gated, iter, st); break;
-    case 4: launch_build_t<true, false, false>(d, nw, gated, iter, st); break;
-    case 5: launch_build_t<true, false, true>(d, nw, gated, iter, st); break;
-    case 6: launch_build_t<true, true, false>(d, nw, gated, iter, st); break;
-    default: launch_build_t<true, true, true>(d, nw, gated, iter, st); break;
-    }
-}
-
 void launch_angular_order(const FmDev &d, int gated, int iter, cudaStream_t st)
 {
     pdl_launch(k_angular_order, sgrid(d.n, 256, 8), 256, st, d, gated, iter);
@@ -1859,29 +1250,6 @@ int force_blocks(int n, int tpm) { return nblk(n * tpm, FORCE_THREADS); }
 static int all_pairs_lanes(int n) { return n <= 8192 ? 32 : n <= 32768 ? 8 : 1; }
 int all_pairs_blocks(int n) { return nblk((long long)n * all_pairs_lanes(n), AP_THREADS); }
 
-template <int TPM>
-static void launch_force_tpm(const FmDev &d, int record, int mode, cudaStream_t st)
-{
-    const int g = force_blocks(d.n, TPM);
-#define FM_FORCE_CASE(R, M)                                                                     \
-    if (record == R && mode == M) {                                                             \
-        switch (d.precision + 2 * d.mie + 4 * d.solvent) {                                      \
-        case 0: pdl_launch(k_force<TPM, R, M, 0>, g, FORCE_THREADS, st, d); break;                   \
-        case 1: pdl_launch(k_force<TPM, R, M, 1>, g, FORCE_THREADS, st, d); break;                   \
-        case 2: pdl_launch(k_force<TPM, R, M, 2>, g, FORCE_THREADS, st, d); break;                   \
-        case 3: pdl_launch(k_force<TPM, R, M, 3>, g, FORCE_THREADS, st, d); break;                   \
-        case 4: pdl_launch(k_force<TPM, R, M, 4>, g, FORCE_THREADS, st, d); break;                   \
-        case 5: pdl_launch(k_force<TPM, R, M, 5>, g, FORCE_THREADS, st, d); break;                   \
-        case 6: pdl_launch(k_force<TPM, R, M, 6>, g, FORCE_THREADS, st, d); break;                   \
-        default: pdl_launch(k_force<TPM, R, M, 7>, g, FORCE_THREADS, st, d); break;                  \
-        }                                                                                       \
-        return;                                                                                 \
-    }
-    FM_FORCE_CASE(0, 0) FM_FORCE_CASE(0, 1) FM_FORCE_CASE(0, 2) FM_FORCE_CASE(0, 3)
-    FM_FORCE_CASE(1, 0) FM_FORCE_CASE(1, 1) FM_FORCE_CASE(1, 2) FM_FORCE_CASE(1, 3)
-#undef FM_FORCE_CASE
-}
-
 void launch_force(const FmDev &d, int record, int mode, int tpm, cudaStream_t st)
 {
     if (d.tile) {
@@ -1889,13 +1257,8 @@ void launch_force(const FmDev &d, int record, int mode, int tpm, cudaStream_t st
         else launch_force_tile<8>(d, record, mode, st);
         return;
     }
-    switch (tpm) {
-    case 1: launch_force_tpm<1>(d, record, mode, st); break;
-    case 2: launch_force_tpm<2>(d, record, mode, st); break;
-    case 4: launch_force_tpm<4>(d, record, mode, st); break;
-    case 16: launch_force_tpm<16>(d, record, mode, st); break;
-    default: launch_force_tpm<8>(d, record, mode, st); break;
-    }
+    if (d.mie || d.solvent) launch_force_types(d, record, mode, tpm, st);
+    else launch_force_lj(d, record, mode, tpm, st);
 }
 
 void launch_all_pairs(const FmDev &d, int record, int mode, cudaStream_t st)
