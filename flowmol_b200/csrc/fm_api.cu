@@ -220,7 +220,7 @@ static void release(fm_handle *h)
     void *ptrs[] = {d.pos0, d.pos1, d.vx, d.vy, d.vz, d.ax, d.ay, d.az, d.slot_of, d.tvx, d.tvy, d.tvz,
                     d.tax, d.tay, d.taz, d.cell_of, d.cell_count, d.cell_start, d.perm, d.tile_sum, d.nbr, d.nnbr,
                     d.pe, d.vir, d.partial, d.rec, d.sc, h->tpos, h->tuidx, h->glob, h->stage3, d.chain,
-                    d.subchain, d.bflag, d.tchain, d.tsubchain, d.tbflag, d.bnd, d.nbond,
+                    d.subchain, d.bflag, d.tchain, d.tsubchain, d.tbflag, d.bnd, d.nbond, d.bt_key, d.bt_val, d.slot_by_upload,
                     (void *)d.mie_pair, (void *)d.mie_mass, (void *)d.mie_type_up, d.rdx, d.rdy, d.rdz, d.rf6,
                     d.blk_off, d.nbr16, (void *)d.ang_k, (void *)d.ang_t0, d.funcy, d.tfuncy, h->dd_dev,
                     h->dd_sums};
@@ -300,6 +300,7 @@ static void queue_build(fm_handle *h, int gated, int iter)
 {
     if (h->d.tile) { fm::launch_blk_seg(h->d, gated, iter, h->st); h->launches += 1; }
     fm::launch_build_nlist(h->d, gated, iter, h->st);
+    if (h->d.potential_flag == 1) { fm::launch_bonds(h->d, gated, iter, h->st); h->launches += 1; }
     if (h->d.angular) { fm::launch_angular_order(h->d, gated, iter, h->st); h->launches += 1; }
 }
 
@@ -476,6 +477,9 @@ static int create_impl(const fm_params *p, const DdGeom *g, fm_handle **out)
         FM_ALLOC(d.chain, n) FM_ALLOC(d.subchain, n) FM_ALLOC(d.bflag, n)
         FM_ALLOC(d.tchain, n) FM_ALLOC(d.tsubchain, n) FM_ALLOC(d.tbflag, n)
         FM_ALLOC(d.bnd, 4 * n) FM_ALLOC(d.nbond, n)
+        const size_t places = fm::bond_table_size((int)n);
+        d.bt_mask = (unsigned)(places - 1);
+        FM_ALLOC(d.bt_key, places) FM_ALLOC(d.bt_val, places) FM_ALLOC(d.slot_by_upload, n)
     }
     int nb = std::max(std::max(fm::force_blocks(h->cap, 16), fm::all_pairs_blocks(h->cap)), fm::macro_blocks(h->cap));
     nb = std::max(nb, d.tile_nblk);
@@ -501,6 +505,7 @@ static int create_impl(const fm_params *p, const DdGeom *g, fm_handle **out)
     if (d.chain) cudaMemset(d.chain, 0, sizeof(int32_t) * n);
     if (d.subchain) cudaMemset(d.subchain, 0, sizeof(int32_t) * n);
     if (d.bflag) cudaMemset(d.bflag, 0, sizeof(int4) * n);
+    if (d.bt_key) cudaMemset(d.bt_key, 0xff, sizeof(unsigned long long) * ((size_t)d.bt_mask + 1));
     cudaMemset(d.vir, 0, sizeof(double) * n);
     cudaMemset(d.sc, 0, sizeof(fm::FmScalars));
     fm::launch_reset_scalars(d, nullptr);
@@ -601,6 +606,7 @@ extern "C" int fm_upload_monomers(fm_handle *h, const int32_t *chainID, const in
     FM_CUDA(cudaMemcpyAsync(h->d.subchain, subchainID, 4 * n, cudaMemcpyHostToDevice, h->st));
     FM_CUDA(cudaMemcpyAsync(h->d.bflag, bin_bflag, 16 * n, cudaMemcpyHostToDevice, h->st));
     if (h->d.solvent) fm::launch_set_bead_flags(h->d, h->st);
+    fm::launch_bond_table(h->d, h->st);
     FM_CUDA(cudaGetLastError());
     FM_CUDA(cudaStreamSynchronize(h->st));
     return FM_OK;
@@ -1117,7 +1123,8 @@ static bool capture_branch(fm_handle *h, int flip)
     if (cudaStreamGetCaptureInfo(h->cap_st, &cst, nullptr, &g, nullptr, nullptr) != cudaSuccess || !g) return false;
     cudaGraphConditionalHandle cond{};
     if (cudaGraphConditionalHandleCreate(&cond, g, 0, cudaGraphCondAssignDefault) != cudaSuccess) return false;
-    const int body_kernels = 8 + (d.tile ? 1 : 0) + (d.angular ? 1 : 0) + (h->sort_flag ? 1 : 0);
+    const int body_kernels = 8 + (d.tile ? 1 : 0) + (d.potential_flag == 1 ? 1 : 0) + (d.angular ? 1 : 0) +
+                             (h->sort_flag ? 1 : 0);
     fm::launch_decide_graph(d, flip, p.rebuild_criteria, p.fixed_rebuild, h->half_min_delta, cond, body_kernels,
                             h->cap_st);
     if (cudaStreamGetCaptureInfo(h->cap_st, &cst, nullptr, nullptr, &deps, &nd) != cudaSuccess) return false;
@@ -1148,6 +1155,7 @@ static bool capture_branch(fm_handle *h, int flip)
     fm::launch_reorder(d, 1, h->tpos, h->tuidx, h->cap_st2);
     if (d.tile) fm::launch_blk_seg(d, 1, fm::ITER_DEVICE, h->cap_st2);
     fm::launch_build_nlist(d, 1, fm::ITER_DEVICE, h->cap_st2);
+    if (d.potential_flag == 1) fm::launch_bonds(d, 1, fm::ITER_DEVICE, h->cap_st2);
     if (d.angular) fm::launch_angular_order(d, 1, fm::ITER_DEVICE, h->cap_st2);
     fm::pdl_capture = true;
     return cudaStreamEndCapture(h->cap_st2, &body) == cudaSuccess;

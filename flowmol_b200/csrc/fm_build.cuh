@@ -36,13 +36,6 @@
 // instructions and 848 -> 709 us per 1M build (256 unpruned candidates a window,
 // one group and a sector check per append step before).
 //
-// With FENE polymers (POLY) the same scan discovers bonds the way the
-// reference's check_update_adjacentbeadinfo does (linklist.f90:2542-2584): any
-// candidate of the scanned cells -- at any distance -- with the owner's chain
-// whose subchain bit is set in the owner's bin_bflag words (get_bondflag,
-// modules.f90:602-610, 31 bits per word) is a bond partner.  Pruning is off
-// then (a stretched bond is still found, and fails at the force).
-//
 // With TILE the rows hold, instead of the entry bits, the candidate's 16-bit
 // word offset in the tiled force kernel's staging of the owner's block
 // (fm_tile.cuh): the segment's base in that staging (blk_off) plus the
@@ -76,10 +69,6 @@ struct CellSys {
     int32_t *nnbr;
     int maxn;
     int *max_nbr;               // atomicMax of the row lengths
-    // FENE (POLY only)
-    const int32_t *chain, *subchain;
-    const int4 *bflag;
-    int32_t *bnd, *nbond;
     // tiled force path (TILE only): rows of staging offsets
     uint16_t *nbr16;
     int maxn16, tT, tR;
@@ -93,26 +82,23 @@ struct CellSys {
 };
 
 // Per-warp shared staging.
-template <bool POLY, bool TILE = false>
+template <bool TILE = false>
 struct BuildShared {
     float4 f[NB_STAGE];         // x, y, z offsets and the entry bits in w
     alignas(16) float ox[32];   // owners' offsets (+1e30 past the last owner),
     alignas(16) float oy[32];   // read in 8-byte pairs
     alignas(16) float oz[32];
     int oi[32];                 // owners' molecule indices
-    int2 cs[POLY ? NB_STAGE : 1];  // chain, subchain of candidates
     int off[55];                // candidate offset of segment k (54 segments + total)
     int start[54], code[54];
     int lbase[TILE ? 54 : 1];                   // segment k's first candidate in the block staging
     unsigned short loc[TILE ? NB_STAGE : 1];    // staged candidates' staging offsets
     int ring[TILE ? 1 : NB_RING][32];           // entries an owner lane has not written yet (generic rows)
     alignas(16) unsigned short ob16[TILE ? 32 : 1][32];  // (tiled rows, 4 T <= 32 entries)
-    int ochain[POLY ? 32 : 1];
-    alignas(16) int4 obf[POLY ? 32 : 1];
-    unsigned hits[POLY ? 1 : 2][32];  // per owner: which of the 32 candidates hit (polymers: registers)
+    unsigned hits[2][32];  // per owner: which of the 32 candidates of each half hit
 };
 
-constexpr uint32_t BUILD_OVER_LIST = 1u, BUILD_OVER_BONDS = 2u;
+constexpr uint32_t BUILD_OVER_LIST = 1u;
 
 // Packed FP32 pairs (sm_100 f32x2 arithmetic): two owners' distance terms
 // per instruction, each half rounded exactly as the scalar operation.
@@ -238,10 +224,10 @@ __device__ __forceinline__ void append_hits(SH &sh, int lane, unsigned m0, unsig
 }
 
 // Rows of every molecule of cell c (0-based extended index) of system y, by
-// one warp.  Returns BUILD_OVER_* bits when a row or a bond set overflowed
+// one warp.  Returns BUILD_OVER_LIST when a row overflowed
 // (the counts past the capacity are still reported through max_nbr).
-template <bool POLY, bool TILE = false>
-__device__ uint32_t build_cell(const CellSys &y, int c, BuildShared<POLY, TILE> &sh, int lane)
+template <bool TILE = false>
+__device__ uint32_t build_cell(const CellSys &y, int c, BuildShared<TILE> &sh, int lane)
 {
     const int ne0 = y.ne[0], ne1 = y.ne[1], ne2 = y.ne[2];
     const int cstart = y.cell_start[c] - y.mol_off;
@@ -339,7 +325,7 @@ __device__ uint32_t build_cell(const CellSys &y, int c, BuildShared<POLY, TILE> 
         const float bx0 = warp_min(xif), bx1 = warp_max(xif);
         const float by0 = warp_min(yif), by1 = warp_max(yif);
         const float bz0 = warp_min(zif), bz1 = warp_max(zif);
-        int cnt = 0, nb = 0;  // the owner lane's list and bond counts
+        int cnt = 0;          // the owner lane's list count
         int out = 0;          // entries already in the row: whole sectors
         int32_t *const row = TILE ? nullptr : y.nbr + nb_row(i, maxn);
         uint16_t *const row16 = TILE ? y.nbr16 + tile_row16(i, maxn) : nullptr;
@@ -350,10 +336,6 @@ __device__ uint32_t build_cell(const CellSys &y, int c, BuildShared<POLY, TILE> 
         sh.oy[lane] = own ? yif : 1e30f;
         sh.oz[lane] = own ? zif : 1e30f;
         sh.oi[lane] = i;
-        if (POLY) {
-            sh.ochain[lane] = own ? y.chain[i] : -1;
-            sh.obf[lane] = own ? y.bflag[i] : make_int4(0, 0, 0, 0);
-        }
         // Candidates are staged 32 a step, in visiting order; those that cannot
         // lie within rneighbr of some owner of this pass are left out (ballot
         // compaction). Whenever 64 are there, and at the end, the owners test
@@ -385,21 +367,19 @@ __device__ uint32_t build_cell(const CellSys &y, int c, BuildShared<POLY, TILE> 
                     const float ex = fmaxf(fmaxf(bx0 - f.x, f.x - bx1), 0.f);
                     const float ey = fmaxf(fmaxf(by0 - f.y, f.y - by1), 0.f);
                     const float ez = fmaxf(fmaxf(bz0 - f.z, f.z - bz1), 0.f);
-                    keep = POLY || ex * ex + ey * ey + ez * ez < prune2;
+                    keep = ex * ex + ey * ey + ez * ez < prune2;
                 }
                 const unsigned m = __ballot_sync(0xffffffffu, keep);
                 if (keep) {
                     const int pos = kept + __popc(m & lt);
                     sh.f[pos] = f;
                     if (TILE) sh.loc[pos] = (unsigned short)loc;
-                    if (POLY) sh.cs[pos] = make_int2(y.chain[j], y.subchain[j]);
                 }
                 kept += __popc(m);
             }
             __syncwarp();
             if (kept < 64 && t0 + 32 < total) continue;
             do {
-                unsigned mine[2] = {0u, 0u};  // the owner lane's hits among the two halves
 #pragma unroll 1
                 for (int half = 0; 32 * half < min(kept, 64); half++) {
                     const int cq = 32 * half + lane;
@@ -409,9 +389,6 @@ __device__ uint32_t build_cell(const CellSys &y, int c, BuildShared<POLY, TILE> 
                     const int e = __float_as_int(f.w);
                     const unsigned long long fx2 = pack_f32x2(f.x, f.x), fy2 = pack_f32x2(f.y, f.y),
                                              fz2 = pack_f32x2(f.z, f.z);
-                    int2 cs = make_int2(-2, 0);
-                    if (POLY && valid) cs = sh.cs[cq];
-                    unsigned mine_reg = 0u;  // polymers: the owner lane keeps its ballot in a register
                     // owners in groups of NB_OG (pairs in packed FP32): independent chains
                     // for the scheduler
                     for (int o0 = 0; o0 < nown; o0 += NB_OG) {
@@ -431,7 +408,7 @@ __device__ uint32_t build_cell(const CellSys &y, int c, BuildShared<POLY, TILE> 
                         for (int u = 0; u < NB_OG; u++) {
                             // the band around rneighbr2 is decided in FP64; the owner
                             // itself (r2f exactly 0) is a hit here, dropped at the append
-                            hit[u] = r2f[u] < lo32 && (!POLY || r2f[u] > 0.f);
+                            hit[u] = r2f[u] < lo32;
                             exact[u] = !hit[u] && r2f[u] <= hi32;
                             anyx |= exact[u];
                         }
@@ -443,42 +420,14 @@ __device__ uint32_t build_cell(const CellSys &y, int c, BuildShared<POLY, TILE> 
 #pragma unroll
                         for (int u = 0; u < NB_OG; u++) {
                             const unsigned m = __ballot_sync(0xffffffffu, hit[u]);
-                            if (POLY) {
-                                if (lane == o0 + u) mine_reg = m;
-                            } else if (lane == 0) {
-                                sh.hits[half][o0 + u] = m;
-                            }
-                        }
-                        if (POLY) {
-                            int addb = 0;
-#pragma unroll
-                            for (int u = 0; u < NB_OG; u++) {
-                                bool bond = false;
-                                if (valid && o0 + u < nown && cs.x == sh.ochain[o0 + u] &&
-                                    !((e & NB_INDEX_MASK) == sh.oi[o0 + u] && (e >> NB_SHIFT_BITS) == NB_NOSHIFT)) {
-                                    const int pos = cs.y - 1, grp = pos / 31, ex = pos % 31;
-                                    const int4 bf = sh.obf[o0 + u];
-                                    const int word = grp == 0 ? bf.x : grp == 1 ? bf.y : grp == 2 ? bf.z : bf.w;
-                                    bond = pos >= 0 && grp < 4 && ((word >> ex) & 1);
-                                }
-                                const unsigned mb = __ballot_sync(0xffffffffu, bond);
-                                const int b0 = __shfl_sync(0xffffffffu, nb, o0 + u);
-                                if (bond) {
-                                    const int k = b0 + __popc(mb & lt);
-                                    if (k < 4) y.bnd[(size_t)sh.oi[o0 + u] * 4 + k] = e;
-                                }
-                                if (lane == o0 + u) addb = __popc(mb);
-                            }
-                            nb += addb;
+                            if (lane == 0) sh.hits[half][o0 + u] = m;
                         }
                     }
-                    if (POLY) mine[half] = mine_reg;
                 }
-                if (!POLY) {
-                    __syncwarp();
-                    mine[0] = lane < nown && kept > 0 ? sh.hits[0][lane] : 0u;
-                    mine[1] = lane < nown && kept > 32 ? sh.hits[1][lane] : 0u;
-                }
+                __syncwarp();
+                // the owner lane's hits among the two halves
+                const unsigned mine[2] = {lane < nown && kept > 0 ? sh.hits[0][lane] : 0u,
+                                          lane < nown && kept > 32 ? sh.hits[1][lane] : 0u};
                 if constexpr (TILE) {
                     for (int half = 0; half < 2; half++)
                         for (unsigned m = mine[half]; m != 0u; m &= m - 1u) {
@@ -496,7 +445,6 @@ __device__ uint32_t build_cell(const CellSys &y, int c, BuildShared<POLY, TILE> 
                     if (lane < left) {
                         sh.f[lane] = sh.f[64 + lane];
                         if (TILE) sh.loc[lane] = sh.loc[64 + lane];
-                        if (POLY) sh.cs[lane] = sh.cs[64 + lane];
                     }
                     __syncwarp();
                 }
@@ -512,10 +460,6 @@ __device__ uint32_t build_cell(const CellSys &y, int c, BuildShared<POLY, TILE> 
             y.nnbr[i] = cnt < maxn ? cnt : maxn;
             atomicMax(y.max_nbr, cnt);
             if (cnt > maxn) over |= BUILD_OVER_LIST;
-            if (POLY) {
-                y.nbond[i] = nb < 4 ? nb : 4;
-                if (nb > 4) over |= BUILD_OVER_BONDS;  // too_many_bonds_error
-            }
         }
     }
     __syncwarp();
@@ -534,7 +478,7 @@ __device__ uint32_t build_cell(const CellSys &y, int c, BuildShared<POLY, TILE> 
 
 constexpr int NB_BSEG = 128;  // 64 union cells x (real, images)
 
-template <bool POLY, bool TILE = false>
+template <bool TILE = false>
 struct BlockShared {
     float4 f[NB_STAGE];             // candidate offsets from the block centre, entry bits in w
     alignas(16) float ox[32];       // owners (+1e30 past the last owner)
@@ -543,7 +487,6 @@ struct BlockShared {
     int oi[32];
     unsigned oallow[32];            // one-hot bit of the owner's cell in the block, 0 past the last
     unsigned char allow[NB_STAGE];  // owner cells a staged candidate may pair with
-    int2 cs[POLY ? NB_STAGE : 1];
     int off[NB_BSEG + 1];
     int start[NB_BSEG], code[NB_BSEG];
     int lbase[TILE ? NB_BSEG : 1];               // segment k's first candidate in the block staging
@@ -552,13 +495,11 @@ struct BlockShared {
     alignas(16) unsigned short ob16[TILE ? 32 : 1][32];  // (tiled rows, 4 T <= 32 entries)
     unsigned char segallow[NB_BSEG];
     int opre[9], ostart[8];         // owners by block cell: prefix counts, first molecule
-    int ochain[POLY ? 32 : 1];
-    alignas(16) int4 obf[POLY ? 32 : 1];
-    unsigned hits[POLY ? 1 : 2][32];  // per owner: which of the 32 candidates hit (polymers: registers)
+    unsigned hits[2][32];  // per owner: which of the 32 candidates of each half hit
 };
 
-template <bool POLY, bool TILE = false>
-__device__ uint32_t build_block(const CellSys &y, int blk, BlockShared<POLY, TILE> &sh, int lane)
+template <bool TILE = false>
+__device__ uint32_t build_block(const CellSys &y, int blk, BlockShared<TILE> &sh, int lane)
 {
     const int ne0 = y.ne[0], ne1 = y.ne[1], ne2 = y.ne[2];
     const int nb0 = (ne0 + 1) / 2, nb1 = (ne1 + 1) / 2;
@@ -694,7 +635,7 @@ __device__ uint32_t build_block(const CellSys &y, int blk, BlockShared<POLY, TIL
         const float bx_lo = warp_min(own ? xif : 3e38f), bx_hi = warp_max(own ? xif : -3e38f);
         const float by_lo = warp_min(own ? yif : 3e38f), by_hi = warp_max(own ? yif : -3e38f);
         const float bz_lo = warp_min(own ? zif : 3e38f), bz_hi = warp_max(own ? zif : -3e38f);
-        int cnt = 0, nb = 0, out = 0;
+        int cnt = 0, out = 0;
         int32_t *const row = TILE ? nullptr : y.nbr + nb_row(i, maxn);
         uint16_t *const row16 = TILE ? y.nbr16 + tile_row16(i, maxn) : nullptr;
         const int self_e = i | (NB_NOSHIFT << NB_SHIFT_BITS);  // the owner's own entry
@@ -705,10 +646,6 @@ __device__ uint32_t build_block(const CellSys &y, int blk, BlockShared<POLY, TIL
         sh.oz[lane] = own ? zif : 1e30f;
         sh.oi[lane] = i;
         sh.oallow[lane] = own ? 1u << oc : 0u;
-        if (POLY) {
-            sh.ochain[lane] = own ? y.chain[i] : -1;
-            sh.obf[lane] = own ? y.bflag[i] : make_int4(0, 0, 0, 0);
-        }
         // Candidates are staged 32 a step, in visiting order; those that cannot
         // lie within rneighbr of some owner of this pass are left out (ballot
         // compaction). Whenever 64 are there, and at the end, the owners test
@@ -740,7 +677,7 @@ __device__ uint32_t build_block(const CellSys &y, int blk, BlockShared<POLY, TIL
                     const float ex = fmaxf(fmaxf(bx_lo - f.x, f.x - bx_hi), 0.f);
                     const float ey = fmaxf(fmaxf(by_lo - f.y, f.y - by_hi), 0.f);
                     const float ez = fmaxf(fmaxf(bz_lo - f.z, f.z - bz_hi), 0.f);
-                    keep = POLY || ex * ex + ey * ey + ez * ez < prune2;
+                    keep = ex * ex + ey * ey + ez * ez < prune2;
                 }
                 const unsigned m = __ballot_sync(0xffffffffu, keep);
                 if (keep) {
@@ -748,14 +685,12 @@ __device__ uint32_t build_block(const CellSys &y, int blk, BlockShared<POLY, TIL
                     sh.f[pos] = f;
                     sh.allow[pos] = (unsigned char)al;
                     if (TILE) sh.loc[pos] = (unsigned short)loc;
-                    if (POLY) sh.cs[pos] = make_int2(y.chain[j], y.subchain[j]);
                 }
                 kept += __popc(m);
             }
             __syncwarp();
             if (kept < 64 && t0 + 32 < total) continue;
             do {
-                unsigned mine[2] = {0u, 0u};  // the owner lane's hits among the two halves
 #pragma unroll 1
                 for (int half = 0; 32 * half < min(kept, 64); half++) {
                     const int cq = 32 * half + lane;
@@ -765,9 +700,6 @@ __device__ uint32_t build_block(const CellSys &y, int blk, BlockShared<POLY, TIL
                     const int e = __float_as_int(f.w);
                     const unsigned long long fx2 = pack_f32x2(f.x, f.x), fy2 = pack_f32x2(f.y, f.y),
                                              fz2 = pack_f32x2(f.z, f.z);
-                    int2 cs = make_int2(-2, 0);
-                    if (POLY && valid) cs = sh.cs[cq];
-                    unsigned mine_reg = 0u;  // polymers: the owner lane keeps its ballot in a register
                     for (int o0 = 0; o0 < nown; o0 += NB_OG) {
                         bool hit[NB_OG], exact[NB_OG];
                         float r2f[NB_OG];
@@ -784,8 +716,8 @@ __device__ uint32_t build_block(const CellSys &y, int blk, BlockShared<POLY, TIL
 #pragma unroll
                         for (int u = 0; u < NB_OG; u++) {
                             const bool ok = (callow & sh.oallow[o0 + u]) != 0u;
-                            // the owner itself: dropped at the append (polymers: decided in FP64)
-                            hit[u] = ok && r2f[u] < lo32 && (!POLY || r2f[u] > 0.f);
+                            // the owner itself: dropped at the append
+                            hit[u] = ok && r2f[u] < lo32;
                             exact[u] = ok && !hit[u] && r2f[u] <= hi32;
                             anyx |= exact[u];
                         }
@@ -797,42 +729,14 @@ __device__ uint32_t build_block(const CellSys &y, int blk, BlockShared<POLY, TIL
 #pragma unroll
                         for (int u = 0; u < NB_OG; u++) {
                             const unsigned m = __ballot_sync(0xffffffffu, hit[u]);
-                            if (POLY) {
-                                if (lane == o0 + u) mine_reg = m;
-                            } else if (lane == 0) {
-                                sh.hits[half][o0 + u] = m;
-                            }
-                        }
-                        if (POLY) {
-                            int addb = 0;
-#pragma unroll
-                            for (int u = 0; u < NB_OG; u++) {
-                                bool bond = false;
-                                if ((callow & sh.oallow[o0 + u]) != 0u && cs.x == sh.ochain[o0 + u] &&
-                                    !((e & NB_INDEX_MASK) == sh.oi[o0 + u] && (e >> NB_SHIFT_BITS) == NB_NOSHIFT)) {
-                                    const int pos = cs.y - 1, grp = pos / 31, ex = pos % 31;
-                                    const int4 bf = sh.obf[o0 + u];
-                                    const int word = grp == 0 ? bf.x : grp == 1 ? bf.y : grp == 2 ? bf.z : bf.w;
-                                    bond = pos >= 0 && grp < 4 && ((word >> ex) & 1);
-                                }
-                                const unsigned mb = __ballot_sync(0xffffffffu, bond);
-                                const int b0 = __shfl_sync(0xffffffffu, nb, o0 + u);
-                                if (bond) {
-                                    const int kb = b0 + __popc(mb & lt);
-                                    if (kb < 4) y.bnd[(size_t)sh.oi[o0 + u] * 4 + kb] = e;
-                                }
-                                if (lane == o0 + u) addb = __popc(mb);
-                            }
-                            nb += addb;
+                            if (lane == 0) sh.hits[half][o0 + u] = m;
                         }
                     }
-                    if (POLY) mine[half] = mine_reg;
                 }
-                if (!POLY) {
-                    __syncwarp();
-                    mine[0] = lane < nown && kept > 0 ? sh.hits[0][lane] : 0u;
-                    mine[1] = lane < nown && kept > 32 ? sh.hits[1][lane] : 0u;
-                }
+                __syncwarp();
+                // the owner lane's hits among the two halves
+                const unsigned mine[2] = {lane < nown && kept > 0 ? sh.hits[0][lane] : 0u,
+                                          lane < nown && kept > 32 ? sh.hits[1][lane] : 0u};
                 if constexpr (TILE) {
                     for (int half = 0; half < 2; half++)
                         for (unsigned m = mine[half]; m != 0u; m &= m - 1u) {
@@ -851,7 +755,6 @@ __device__ uint32_t build_block(const CellSys &y, int blk, BlockShared<POLY, TIL
                         sh.f[lane] = sh.f[64 + lane];
                         sh.allow[lane] = sh.allow[64 + lane];
                         if (TILE) sh.loc[lane] = sh.loc[64 + lane];
-                        if (POLY) sh.cs[lane] = sh.cs[64 + lane];
                     }
                     __syncwarp();
                 }
@@ -867,10 +770,6 @@ __device__ uint32_t build_block(const CellSys &y, int blk, BlockShared<POLY, TIL
             y.nnbr[i] = cnt < maxn ? cnt : maxn;
             atomicMax(y.max_nbr, cnt);
             if (cnt > maxn) over |= BUILD_OVER_LIST;
-            if (POLY) {
-                y.nbond[i] = nb < 4 ? nb : 4;
-                if (nb > 4) over |= BUILD_OVER_BONDS;
-            }
         }
     }
     __syncwarp();

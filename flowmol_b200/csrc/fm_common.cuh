@@ -123,6 +123,12 @@ struct FmDev {
     int32_t *tchain, *tsubchain;
     int4 *tbflag;
     int32_t *bnd, *nbond;
+    // beads by (chain, subchain), fm_bonds.cu: open addressing, keys and upload
+    // indices; and the slot of each upload index
+    unsigned long long *bt_key;
+    int32_t *bt_val;
+    unsigned bt_mask;
+    int32_t *slot_by_upload;
     // Mie_potential 1: per-type-pair constants, per-type masses; a molecule's
     // type (1-based) rides in the w component of its position
     int build_rows;              // list build by molecule (fm_rows.cuh); else by warp, build_blocks choosing
@@ -259,9 +265,13 @@ void launch_scatter(const FmDev &d, int gated, cudaStream_t st);
 void launch_reorder(const FmDev &d, int gated, double4 *tpos, int32_t *tuidx, cudaStream_t st);
 void launch_build_nlist(const FmDev &d, int gated, int iter, cudaStream_t st);
 // The same rows by molecule (fm_rows.cu), for up to ROWS_MAX_MOLECULES: 32,000
-// molecules 78 us against ~130 by warp, 108,000 264 against 160.
+// molecules 64 us against ~130 by warp, 108,000 170 against 160.
 constexpr int ROWS_MAX_MOLECULES = 65536;
 void launch_rows(const FmDev &d, int gated, int iter, cudaStream_t st);
+// Bonds (potential_flag 1): the bead table at upload, the bonds after each build.
+size_t bond_table_size(int n);
+void launch_bond_table(const FmDev &d, cudaStream_t st);
+void launch_bonds(const FmDev &d, int gated, int iter, cudaStream_t st);
 // angular_potential: orders each middle bead's two bonds as the reference's
 // list build discovers them (after every build).
 void launch_angular_order(const FmDev &d, int gated, int iter, cudaStream_t st);

@@ -140,6 +140,65 @@ __device__ __forceinline__ double4 ldg_pos(const double4 *p)
     return r;
 }
 
+// Sorts perm[b .. b+m) by key(perm value), by one warp: up to 32 members by a
+// bitonic sort in registers (as many stages as they need), up to 128 by rank,
+// more by lane 0 (insertion). Keys are distinct and below 2^59.
+constexpr int SORT_RANK = 128;
+template <typename K>
+__device__ __forceinline__ void warp_sort_cell(int32_t *perm, int b, int m, int lane, K &&key_of)
+{
+    if (m <= 1) return;
+    if (m <= 32) {
+        unsigned long long key = ~0ull;
+        int o = 0;
+        if (lane < m) {
+            o = perm[b + lane];
+            key = key_of(o) << 5 | (unsigned)lane;
+        }
+        for (int k = 2; k < 2 * m; k <<= 1) {
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, j);
+                const bool keep_min = ((lane & j) == 0) == ((lane & k) == 0);
+                key = keep_min ? (key < other ? key : other) : (key > other ? key : other);
+            }
+        }
+        o = __shfl_sync(0xffffffffu, o, (int)(key & 31u));
+        if (lane < m) perm[b + lane] = o;
+    } else if (m <= SORT_RANK) {
+        unsigned long long key[SORT_RANK / 32];
+        int o[SORT_RANK / 32], rank[SORT_RANK / 32];
+#pragma unroll
+        for (int q = 0; q < SORT_RANK / 32; q++) {
+            const int x = q * 32 + lane;
+            o[q] = x < m ? perm[b + x] : 0;
+            key[q] = x < m ? key_of(o[q]) : ~0ull;
+            rank[q] = 0;
+        }
+#pragma unroll
+        for (int p = 0; p < SORT_RANK / 32; p++)
+            for (int l = 0; l < 32; l++) {
+                const unsigned long long other = __shfl_sync(0xffffffffu, key[p], l);
+#pragma unroll
+                for (int q = 0; q < SORT_RANK / 32; q++) rank[q] += other < key[q] ? 1 : 0;
+            }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < SORT_RANK / 32; q++)
+            if (q * 32 + lane < m) perm[b + rank[q]] = o[q];
+    } else if (lane == 0) {
+        for (int x = b + 1; x < b + m; x++) {
+            const int o = perm[x];
+            const unsigned long long key = key_of(o);
+            int y = x - 1;
+            while (y >= b && key_of(perm[y]) > key) {
+                perm[y + 1] = perm[y];
+                y--;
+            }
+            perm[y + 1] = o;
+        }
+    }
+}
+
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v)
 {

@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "fm_engine.cuh"
+#include "fm_rows.cuh"
 #include "flowmol_b200.h"
 
 namespace {
@@ -158,7 +159,7 @@ void free_all(fm_engine *e)
     void *ptrs[] = {d.slots, d.flags, d.pos0, d.pos1, d.vx, d.vy, d.vz, d.ax, d.ay, d.az, d.slot_of, d.uidx, d.tag,
                     d.rteth, d.slidev, d.tpos, d.trteth, d.tslidev, d.tvx, d.tvy, d.tvz, d.tax, d.tay, d.taz,
                     d.tuidx, d.ttag, d.cell_slot, d.cell_of, d.cell_count, d.cell_start, d.perm, d.nbr, d.nnbr,
-                    d.rterm, d.tmv2, d.red_part, d.red_count, d.rb_slot, d.rb_mpre, d.rb_cpre, d.rb_upre, e->stage,
+                    d.rterm, d.tmv2, d.red_part, d.red_count, d.rb_slot, d.rb_mpre, d.rb_cpre, d.rb_upre, d.rb_rpre, e->stage,
                     e->stage_i};
     for (void *q : ptrs)
         if (q) cudaFree(q);
@@ -226,7 +227,7 @@ bool capture_loop(fm_engine *e)
                  cudaSuccess;
             if (ok) {
                 const int k = loop_body_ticks(e);
-                for (int t = 0; t < k; t++) fm::eng_tick(e->d, e->tpm, e->need_x, e->cap_st);
+                for (int t = 0; t < k; t++) fm::eng_tick(e->d, e->tpm, e->need_x, t == 0, e->cap_st);
                 fm::eng_loop_continue(e->d, e->need_x.slots, cond, k, std::max(e->p.ticks_per_chunk, 1),
                                       e->cap_st);
                 ok = cudaStreamEndCapture(e->cap_st, &body) == cudaSuccess;
@@ -259,7 +260,7 @@ int capture(fm_engine *e)
     if (capture_loop(e)) return FM_OK;
     cudaGraph_t g;
     EN_CUDA(cudaStreamBeginCapture(e->st, cudaStreamCaptureModeThreadLocal));
-    for (int t = 0; t < e->p.ticks_per_chunk; t++) fm::eng_tick(e->d, e->tpm, e->need_x, e->st);
+    for (int t = 0; t < e->p.ticks_per_chunk; t++) fm::eng_tick(e->d, e->tpm, e->need_x, t == 0, e->st);
     cudaError_t err = cudaStreamEndCapture(e->st, &g);
     if (err != cudaSuccess) return efail(FM_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(err));
     err = cudaGraphInstantiate(&e->graph, g, 0);
@@ -365,6 +366,7 @@ int admit(fm_engine *e, Job &jb, int slot)
     s.maxn = jb.maxn;
     // sparse cells (a few molecules each) are built 2x2x2 at a time (same rows);
     // the threshold is the autotuner's
+    s.rows_g = f.mode == fm::MODE_LIST ? fm::rows_lanes(per_cell(s, j.np)) : 32;
     s.build_blocks = f.mode == fm::MODE_LIST && per_cell(s, j.np) < e->blocks_below ? 1 : 0;
     s.tplot = std::max(1, j.tplot);
     s.integrator = j.integration_algorithm == 0 ? 0 : 1;
@@ -537,6 +539,7 @@ int tune_build(fm_engine *e)
         fl.any_rebuild = 1;
         fl.rb_n = (int)ks.size();
         fl.rb_utot = tot;
+        fl.rb_rows = 0;  // the tile of the build by warp
         cudaError_t ce = cudaMemcpyAsync(sslots, tmp.data(), sizeof(fm::EngSlot) * tmp.size(),
                                          cudaMemcpyHostToDevice, e->st);
         if (ce == cudaSuccess)
@@ -697,7 +700,7 @@ extern "C" int fm_engine_create(const fm_engine_params *p, fm_engine **out)
     EA(d.perm, M) EA(d.nbr, p->max_list_entries) EA(d.nnbr, M) EA(d.rterm, M * fm::RT_N) EA(d.tmv2, M)
     EA(d.red_part, (size_t)d.nslots * fm::EY * fm::RED_W) EA(d.red_count, (size_t)d.nslots * 2)
     EA(d.rb_slot, (size_t)d.nslots + 1) EA(d.rb_mpre, (size_t)d.nslots + 1) EA(d.rb_cpre, (size_t)d.nslots + 1)
-    EA(d.rb_upre, (size_t)d.nslots + 1)
+    EA(d.rb_upre, (size_t)d.nslots + 1) EA(d.rb_rpre, (size_t)d.nslots + 1)
 #undef EA
     if (rc != FM_OK) {
         free_all(e);
@@ -726,6 +729,7 @@ extern "C" int fm_engine_create(const fm_engine_params *p, fm_engine **out)
     e->resident.assign((size_t)p->max_slots, Job());
     e->table.assign((size_t)p->max_slots, fm::EngSlot{});
     e->tpm = p->threads_per_molecule > 0 ? p->threads_per_molecule : 4;
+    d.rows_ok = p->list_build == FM_LIST_BUILD_AUTO ? 1 : 0;
     e->blocks_below = p->list_build == FM_LIST_BUILD_CELLS ? 0.0 : (p->list_build == FM_LIST_BUILD_BLOCKS ? 1e30 : 8.0);
     cudaError_t err = cudaDeviceSynchronize();
     if (err != cudaSuccess) {
@@ -825,7 +829,7 @@ extern "C" int fm_engine_step_chunk(fm_engine *e, int32_t *resident_out, int32_t
             // that the autotuner times them running before the tick loop --
             // which may run a whole batch in one launch -- is captured with its
             // choice
-            fm::eng_tick(e->d, e->tpm, e->need_x, e->st);
+            fm::eng_tick(e->d, e->tpm, e->need_x, true, e->st);
             e->ticks += 1;
             e->launches += fm::eng_kernels_per_tick();
             EN_TRY(sync_table(e));

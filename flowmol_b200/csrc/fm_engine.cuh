@@ -33,7 +33,8 @@ struct EngSlot {
     int mol_off, nmol;                // molecules [mol_off, +nmol)
     int64_t list_off;                 // neighbour rows start here, maxn entries per molecule
     int maxn;
-    int build_blocks;                 // list build by 2x2x2 cells (sparse jobs), else by cell
+    int build_blocks;                 // list build by warp: by 2x2x2 cells (sparse jobs), else by cell
+    int rows_g;                       // list build by molecule: lanes per molecule (rows_lanes)
     int tplot, integrator, ensemble, mode, pressure, nthermo, crit, fixed_rebuild;
     int iter0, nsteps;
     double rc2, rn2, potshift, half_min_delta, volume, density;
@@ -45,7 +46,8 @@ struct EngSlot {
     uint32_t status;
     int fail_iter;
     int rebuilds, nsamples;
-    int max_nbr, pad_;
+    int max_nbr;
+    int strays;                       // last cell sort: a real molecule is binned in a halo cell
     unsigned long long vmax2;
     double rmax, simtime;
     double zeta[2], ascale[2], bscale[2];
@@ -62,6 +64,8 @@ struct EngFlags {
     // this tick's rebuilding jobs (slot order): count, their molecules, their
     // cells, their list-build units (cells or 2x2x2 blocks)
     int rb_n, rb_mtot, rb_ctot, rb_utot;
+    // list build by molecule this tick (fm_rows.cuh), and its units (warps)
+    int rb_rows, rb_rtot;
     // ticks run by the current launch of the tick loop (the graph's WHILE node),
     // and whether jobs wait in the host's queue (written before each launch)
     int loop_ticks, queue_waiting;
@@ -105,7 +109,9 @@ struct EngDev {
     int32_t *red_count;
     // rebuild work list of the tick: slots, and prefix sums of their molecules
     // and cells ([rb_n + 1] each), so the rebuild kernels visit only those
-    int32_t *rb_slot, *rb_mpre, *rb_cpre, *rb_upre;
+    int32_t *rb_slot, *rb_mpre, *rb_cpre, *rb_upre, *rb_rpre;
+    // list_build automatic: ticks that rebuild few molecules build by molecule
+    int rows_ok;
 };
 
 constexpr int EY = 16;      // blocks per job in the thermostat and record reductions
@@ -122,7 +128,8 @@ struct TickExtent {
 };
 
 // Launchers (fm_engine.cu); `tpm` = lanes per molecule of the force kernel.
-void eng_tick(const EngDev &d, int tpm, const TickExtent &x, cudaStream_t st);
+// `first`: the first kernel of the graph being captured.
+void eng_tick(const EngDev &d, int tpm, const TickExtent &x, bool first, cudaStream_t st);
 // The list build of the work list in d.flags / d.rb_* (autotuner timing runs).
 void eng_build_only(const EngDev &d, int cells, cudaStream_t st);
 void eng_force_only(const EngDev &d, int tpm, int mols, cudaStream_t st);  // autotuner: forces of running list jobs

@@ -31,6 +31,7 @@
 #include "fm_device.cuh"
 #include "fm_engine.cuh"
 #include "fm_build.cuh"
+#include "fm_rows.cuh"
 
 namespace fm {
 
@@ -120,6 +121,7 @@ __device__ __forceinline__ bool slot_rebuilding(const EngSlot &s) { return slot_
 constexpr int EDEC = 1024;
 __global__ void __launch_bounds__(EDEC) k_e_decide(EngDev d)
 {
+    pdl_enter();
     __shared__ int f[6];
     if (threadIdx.x < 6) f[threadIdx.x] = 0;
     __syncthreads();
@@ -141,14 +143,14 @@ __global__ void __launch_bounds__(EDEC) k_e_decide(EngDev d)
         d.flags->any_lfv = f[3]; d.flags->any_thermo = f[4]; d.flags->any_record = f[5];
     }
     // rebuild work list in slot order: a block scan of (flag, molecules, cells)
-    __shared__ int wsum[4][EDEC / 32];
-    __shared__ int carry[4];
-    if (threadIdx.x < 4) carry[threadIdx.x] = 0;
+    __shared__ int wsum[5][EDEC / 32];
+    __shared__ int carry[5];
+    if (threadIdx.x < 5) carry[threadIdx.x] = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int base = 0; base < d.nslots; base += EDEC) {
         const int k = base + threadIdx.x;
-        int x[4] = {0, 0, 0, 0};
+        int x[5] = {0, 0, 0, 0, 0};
         if (k < d.nslots) {
             const EngSlot &s = d.slots[k];
             if (slot_rebuilding(s)) {
@@ -158,11 +160,12 @@ __global__ void __launch_bounds__(EDEC) k_e_decide(EngDev d)
                 x[3] = s.mode != MODE_LIST ? 0
                        : s.build_blocks ? ((s.ne[0] + 1) / 2) * ((s.ne[1] + 1) / 2) * ((s.ne[2] + 1) / 2)
                                         : s.ncell;
+                x[4] = s.mode == MODE_LIST ? (s.nmol + 32 / s.rows_g - 1) / (32 / s.rows_g) : 0;
             }
         }
-        int incl[4];
+        int incl[5];
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
+        for (int q = 0; q < 5; q++) {
             incl[q] = x[q];
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -174,7 +177,7 @@ __global__ void __launch_bounds__(EDEC) k_e_decide(EngDev d)
         __syncthreads();
         if (w == 0) {
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
+            for (int q = 0; q < 5; q++) {
                 const int v = wsum[q][lane];
                 int vi = v;
 #pragma unroll
@@ -192,16 +195,20 @@ __global__ void __launch_bounds__(EDEC) k_e_decide(EngDev d)
             d.rb_mpre[pos] = carry[1] + wsum[1][w] + incl[1] - x[1];
             d.rb_cpre[pos] = carry[2] + wsum[2][w] + incl[2] - x[2];
             d.rb_upre[pos] = carry[3] + wsum[3][w] + incl[3] - x[3];
+            d.rb_rpre[pos] = carry[4] + wsum[4][w] + incl[4] - x[4];
         }
         __syncthreads();
         if (threadIdx.x == EDEC - 1)
-            for (int q = 0; q < 4; q++) carry[q] += wsum[q][w] + incl[q];
+            for (int q = 0; q < 5; q++) carry[q] += wsum[q][w] + incl[q];
         __syncthreads();
     }
     if (threadIdx.x == 0) {
         d.rb_mpre[carry[0]] = carry[1];
         d.rb_cpre[carry[0]] = carry[2];
         d.rb_upre[carry[0]] = carry[3];
+        d.rb_rpre[carry[0]] = carry[4];
+        d.flags->rb_rtot = carry[4];
+        d.flags->rb_rows = d.rows_ok && carry[1] <= ROWS_MAX_MOLECULES;
         d.flags->rb_n = carry[0];
         d.flags->rb_mtot = carry[1];
         d.flags->rb_ctot = carry[2];
@@ -224,6 +231,7 @@ __device__ __forceinline__ int rb_entry(const int32_t *pre, int g, int &r)
 
 __global__ void k_e_wrap_bin(EngDev d)
 {
+    pdl_enter();
     if (!d.flags->any_rebuild) return;
     const int tot = d.flags->rb_mtot;
     int r = 0;
@@ -267,12 +275,13 @@ __global__ void k_e_wrap_bin(EngDev d)
 constexpr int ESCAN = 1024;
 __global__ void __launch_bounds__(ESCAN) k_e_scan(EngDev d)
 {
+    pdl_enter();
     if (!d.flags->any_rebuild) return;
-    const EngSlot &s = d.slots[blockIdx.x];
+    EngSlot &s = d.slots[blockIdx.x];
     if (!slot_rebuilding(s) || s.mode != MODE_LIST) return;
     __shared__ int ws[ESCAN / 32];
     __shared__ int carry_s;
-    if (threadIdx.x == 0) carry_s = s.mol_off;
+    if (threadIdx.x == 0) { carry_s = s.mol_off; s.strays = 0; }
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int base = 0; base < s.ncell; base += ESCAN) {
@@ -310,6 +319,7 @@ __global__ void __launch_bounds__(ESCAN) k_e_scan(EngDev d)
 
 __global__ void k_e_scatter(EngDev d)
 {
+    pdl_enter();
     if (!d.flags->any_rebuild) return;
     const int tot = d.flags->rb_mtot;
     int r = 0;
@@ -324,31 +334,34 @@ __global__ void k_e_scatter(EngDev d)
     }
 }
 
+// Cell by cell, one warp each: by octant, then by the order the molecules had
+// (the single-system cell sort, fm_kernels.cu, goes by identity instead).
 __global__ void k_e_sort(EngDev d)
 {
+    pdl_enter();
     if (!d.flags->any_rebuild) return;
-    const int tot = d.flags->rb_ctot;
+    const int tot = d.flags->rb_ctot, lane = threadIdx.x & 31;
     int r = 0;
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < tot; g += gridDim.x * blockDim.x) {
+    for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < tot; g += (gridDim.x * blockDim.x) >> 5) {
         const int lc = rb_entry(d.rb_cpre, g, r);
-        const EngSlot &s = d.slots[d.rb_slot[r]];
+        EngSlot &s = d.slots[d.rb_slot[r]];
         const int c = s.cell_off + lc;
         const int b = d.cell_start[s.cstart_off + lc], e = d.cell_start[s.cstart_off + lc + 1];
-        for (int x = b + 1; x < e; x++) {
-            int key = d.perm[x];
-            int y = x - 1;
-            while (y >= b && d.perm[y] > key) {
-                d.perm[y + 1] = d.perm[y];
-                y--;
-            }
-            d.perm[y + 1] = key;
-        }
-        d.cell_count[c] = 0;
+        if (lane == 0) d.cell_count[c] = 0;
+        if (b == e) continue;
+        const double4 *P = eng_pos(d, s.pset);
+        const int cx = lc % s.ne[0], cy = (lc / s.ne[0]) % s.ne[1], cz = lc / (s.ne[0] * s.ne[1]);
+        warp_sort_cell(d.perm, b, e - b, lane, [&](int o) {
+            return (unsigned long long)sub_cell(P[o], cx, cy, cz, s.hd, s.cs) << 32 | (unsigned)o;
+        });
+        for (int k = b + lane; k < e; k += 32) d.cell_of[k] = c;  // by new index from here on
+        if (lane == 0 && (is_halo(cx, s.ne[0]) || is_halo(cy, s.ne[1]) || is_halo(cz, s.ne[2]))) s.strays = 1;
     }
 }
 
 __global__ void k_e_reorder_gather(EngDev d)
 {
+    pdl_enter();
     if (!d.flags->any_rebuild) return;
     const int tot = d.flags->rb_mtot;
     int r = 0;
@@ -370,6 +383,7 @@ __global__ void k_e_reorder_gather(EngDev d)
 
 __global__ void k_e_reorder_copy(EngDev d)
 {
+    pdl_enter();
     if (!d.flags->any_rebuild) return;
     const int tot = d.flags->rb_mtot;
     int r = 0;
@@ -388,24 +402,49 @@ __global__ void k_e_reorder_copy(EngDev d)
     }
 }
 
-// Neighbour rows of the tick's rebuilding jobs, one warp per work unit (a
-// cell, or a block of 2x2x2 cells for sparse jobs): the single-system
-// routines (build_cell / build_block, fm_build.cuh: pair set of
-// assign_to_neighbourlist_halfint_opt, linklist.f90:660-804) on the unit's job.
+// One warp's unit of the build by molecule: 32 / G molecules of job s.
+template <int G>
+__device__ __forceinline__ void rows_unit(const EngDev &d, EngSlot &s, const CellSys &y, int unit, RowsShared<G> &sh)
+{
+    const int i = unit * (32 / G) + (int)(threadIdx.x & 31) / G, g = threadIdx.x % G;
+    int cnt = 0;
+    if (i < s.nmol) {
+        cnt = rows_build<G>(y, i, d.cell_of[s.mol_off + i] - s.cell_off, s.strays != 0, g, sh);
+        if (g == 0) y.nnbr[i] = min(cnt, y.maxn);
+    }
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
+    if ((threadIdx.x & 31) == 0) {
+        if (most > *(volatile int *)&s.max_nbr) atomicMax(&s.max_nbr, most);
+        if (most > y.maxn) slot_fail(&s, ST_NLIST, s.iter);
+    }
+}
+
+// Neighbour rows of the tick's rebuilding jobs with the single-system routines
+// (pair set of assign_to_neighbourlist_halfint_opt, linklist.f90:660-804) on
+// the unit's job.  A tick that rebuilds few molecules builds by molecule
+// (rows_build, fm_rows.cuh; unit: a warp's molecules), a larger one by warp
+// (build_cell / build_block, fm_build.cuh; unit: a cell, or a block of 2x2x2
+// cells for sparse jobs).
 __global__ void __launch_bounds__(NB_THREADS, 6) k_e_build(EngDev d)
 {
+    pdl_enter();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     union WarpShared {
-        BuildShared<false> cell;
-        BlockShared<false> block;
+        BuildShared<> cell;
+        BlockShared<> block;
+        RowsShared<8> rows8;
+        RowsShared<16> rows16;
+        RowsShared<32> rows32;
     };
     __shared__ WarpShared sh[NB_WARPS];
     __shared__ CellSys ys[NB_WARPS];  // the unit's job, read through shared memory
     if (!d.flags->any_rebuild) return;
-    const int tot = d.flags->rb_utot;
+    const bool rows = d.flags->rb_rows != 0;
+    const int tot = rows ? d.flags->rb_rtot : d.flags->rb_utot;
+    const int32_t *pre = rows ? d.rb_rpre : d.rb_upre;
     int r = 0, r_loaded = -1;
     for (int g = blockIdx.x * NB_WARPS + warp; g < tot; g += gridDim.x * NB_WARPS) {
-        const int unit = rb_entry(d.rb_upre, g, r);
+        const int unit = rb_entry(pre, g, r);
         EngSlot &s = d.slots[d.rb_slot[r]];
         __syncwarp();
         if (r != r_loaded && lane == 0) {
@@ -419,17 +458,21 @@ __global__ void __launch_bounds__(NB_THREADS, 6) k_e_build(EngDev d)
             y.nnbr = d.nnbr + s.mol_off;
             y.maxn = s.maxn;
             y.max_nbr = &s.max_nbr;
-            y.chain = y.subchain = nullptr;
-            y.bflag = nullptr;
-            y.bnd = y.nbond = nullptr;
             y.dd = 0;
             y.org[0] = y.org[1] = y.org[2] = 0;
         }
         __syncwarp();
         r_loaded = r;
+        const CellSys y = ys[warp];  // in registers: every store to the staging would reload it
+        if (rows) {
+            if (s.rows_g == 8) rows_unit(d, s, y, unit, sh[warp].rows8);
+            else if (s.rows_g == 16) rows_unit(d, s, y, unit, sh[warp].rows16);
+            else rows_unit(d, s, y, unit, sh[warp].rows32);
+            continue;
+        }
         // a cell or, for sparse jobs, a block of 2x2x2 cells: the same rows
-        const uint32_t over = s.build_blocks ? build_block<false>(ys[warp], unit, sh[warp].block, lane)
-                                             : build_cell<false>(ys[warp], unit, sh[warp].cell, lane);
+        const uint32_t over = s.build_blocks ? build_block<false>(y, unit, sh[warp].block, lane)
+                                             : build_cell<false>(y, unit, sh[warp].cell, lane);
         if (lane == 0 && (over & BUILD_OVER_LIST)) slot_fail(&s, ST_NLIST, s.iter);
     }
 }
@@ -563,6 +606,7 @@ constexpr int EF_THREADS = 256;
 template <int TPM, int PREC, bool FORCE_ONLY, bool REC>
 __global__ void __launch_bounds__(EF_THREADS, REC ? 2 : 4) k_e_force(EngDev d)
 {
+    pdl_enter();
     constexpr int PER_BLOCK = EF_THREADS / TPM;
     const int lane = threadIdx.x % TPM;
     if (!FORCE_ONLY && !d.flags->any_list) return;
@@ -636,6 +680,7 @@ constexpr int EAP_XBLOCKS = 32, EAP_YBLOCKS = 16;
 template <int PREC>
 __global__ void __launch_bounds__(EAP_THREADS) k_e_force_ap(EngDev d)
 {
+    pdl_enter();
     if (!d.flags->any_ap) return;
     for (int k = blockIdx.x; k < d.nslots; k += gridDim.x) {
     const EngSlot &s = d.slots[k];
@@ -700,12 +745,15 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double (&c)[NV])
         if (l == 0) { sv[k][w] = v[k]; sc[k][w] = c[k]; }
     }
     __syncthreads();
+    if (threadIdx.x < NV) {
+        double s = sv[threadIdx.x][0], cc = sc[threadIdx.x][0];
+        for (int q = 1; q < ER / 32; q++) nmerge(s, cc, sv[threadIdx.x][q], sc[threadIdx.x][q]);
+        sv[threadIdx.x][0] = s; sc[threadIdx.x][0] = cc;
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
-        for (int k = 0; k < NV; k++) {
-            double s = sv[k][0], cc = sc[k][0];
-            for (int q = 1; q < ER / 32; q++) nmerge(s, cc, sv[k][q], sc[k][q]);
-            v[k] = s; c[k] = cc;
-        }
+#pragma unroll
+        for (int k = 0; k < NV; k++) { v[k] = sv[k][0]; c[k] = sc[k][0]; }
     }
     __syncthreads();
 }
@@ -721,7 +769,10 @@ __device__ __forceinline__ void job_chunk(const EngSlot &s, int y, int &lo, int 
 // Publishes block y's NV compensated sums (and a max) for slot k; the last of
 // the EY blocks to arrive merges all partials in y order into (v, c, mx) and
 // returns true (in thread 0 only).  The merge order does not depend on which
-// block arrives last, so the result is deterministic.
+// block arrives last, so the result is deterministic.  The last block reads
+// all partials at once and a thread per sum merges them: one thread reading and
+// merging them in turn waited for EY x (2 NV + 1) loads, 26 us a tick of the
+// thermostat and 62 us of a record.
 template <int NV>
 __device__ bool job_merge(const EngDev &d, int k, int which, double (&v)[NV], double (&c)[NV], double &mx)
 {
@@ -735,16 +786,28 @@ __device__ bool job_merge(const EngDev &d, int k, int which, double (&v)[NV], do
         last = prev == EY - 1;
     }
     __syncthreads();
-    if (!last || threadIdx.x != 0) return false;
+    if (!last) return false;  // uniform across the block
     __threadfence();
-    const volatile double *all = d.red_part + (size_t)k * EY * RED_W;
-    for (int q = 0; q < NV; q++) { v[q] = all[2 * q]; c[q] = all[2 * q + 1]; }
-    mx = all[2 * NV];
-    for (int y = 1; y < EY; y++) {
-        const volatile double *py = all + (size_t)y * RED_W;
-        for (int q = 0; q < NV; q++) nmerge(v[q], c[q], py[2 * q], py[2 * q + 1]);
-        mx = fmax(mx, py[2 * NV]);
+    __shared__ double all[EY][2 * NV + 1];
+    const double *from = d.red_part + (size_t)k * EY * RED_W;
+    for (int q = threadIdx.x; q < EY * (2 * NV + 1); q += ER)
+        all[q / (2 * NV + 1)][q % (2 * NV + 1)] = __ldcg(from + (size_t)(q / (2 * NV + 1)) * RED_W + q % (2 * NV + 1));
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        const int q = threadIdx.x;
+        double s = all[0][2 * q], cc = all[0][2 * q + 1];
+        for (int y = 1; y < EY; y++) nmerge(s, cc, all[y][2 * q], all[y][2 * q + 1]);
+        all[0][2 * q] = s; all[0][2 * q + 1] = cc;
+    } else if (threadIdx.x == NV) {
+        double m = all[0][2 * NV];
+        for (int y = 1; y < EY; y++) m = fmax(m, all[y][2 * NV]);
+        all[0][2 * NV] = m;
     }
+    __syncthreads();
+    if (threadIdx.x != 0) return false;
+#pragma unroll
+    for (int q = 0; q < NV; q++) { v[q] = all[0][2 * q]; c[q] = all[0][2 * q + 1]; }
+    mx = all[0][2 * NV];
     d.red_count[2 * k + which] = 0;  // ready for the next tick
     return true;
 }
@@ -754,6 +817,7 @@ __device__ bool job_merge(const EngDev &d, int k, int which, double (&v)[NV], do
 // Grid (slot, EY).
 __global__ void __launch_bounds__(ER) k_e_thermo(EngDev d)
 {
+    pdl_enter();
     if (!d.flags->any_thermo) return;
     const int k = blockIdx.x;
     EngSlot &s = d.slots[k];
@@ -783,6 +847,7 @@ __global__ void __launch_bounds__(ER) k_e_thermo(EngDev d)
 
 __global__ void k_e_move_lfv(EngDev d)
 {
+    pdl_enter();
     if (!d.flags->any_lfv) return;
     const int hwm = d.flags->mol_hwm;
     for (int base = blockIdx.x * blockDim.x; base < hwm; base += gridDim.x * blockDim.x) {
@@ -843,6 +908,7 @@ __global__ void k_e_move_lfv(EngDev d)
 // (cumulative_pressure, :3151-3205).  Grid (slot, EY).
 __global__ void __launch_bounds__(ER) k_e_record(EngDev d)
 {
+    pdl_enter();
     if (!d.flags->any_record) return;
     const int k = blockIdx.x;
     EngSlot &s = d.slots[k];
@@ -946,15 +1012,15 @@ void launch_force_t(const EngDev &d, int mols, bool force_only, cudaStream_t st)
 {
     const int g = sgrid((long long)mols * TPM, EF_THREADS, 8);
     if (force_only) {
-        if (d.precision == 0) k_e_force<TPM, 0, true, false><<<g, EF_THREADS, 0, st>>>(d);
-        else k_e_force<TPM, 1, true, false><<<g, EF_THREADS, 0, st>>>(d);
+        if (d.precision == 0) pdl_launch(k_e_force<TPM, 0, true, false>, g, EF_THREADS, st, d);
+        else pdl_launch(k_e_force<TPM, 1, true, false>, g, EF_THREADS, st, d);
     } else {
         if (d.precision == 0) {
-            k_e_force<TPM, 0, false, false><<<g, EF_THREADS, 0, st>>>(d);
-            k_e_force<TPM, 0, false, true><<<g, EF_THREADS, 0, st>>>(d);
+            pdl_launch(k_e_force<TPM, 0, false, false>, g, EF_THREADS, st, d);
+            pdl_launch(k_e_force<TPM, 0, false, true>, g, EF_THREADS, st, d);
         } else {
-            k_e_force<TPM, 1, false, false><<<g, EF_THREADS, 0, st>>>(d);
-            k_e_force<TPM, 1, false, true><<<g, EF_THREADS, 0, st>>>(d);
+            pdl_launch(k_e_force<TPM, 1, false, false>, g, EF_THREADS, st, d);
+            pdl_launch(k_e_force<TPM, 1, false, true>, g, EF_THREADS, st, d);
         }
     }
 }
@@ -1009,31 +1075,37 @@ void eng_loop_continue(const EngDev &d, int slots, cudaGraphConditionalHandle co
     k_e_continue<<<1, 256, 0, st>>>(d, std::min(slots, d.nslots), cond, body_ticks, max_ticks);
 }
 
-void eng_tick(const EngDev &d, int tpm, const TickExtent &x, cudaStream_t st)
+// The kernels of a tick start while their predecessor drains (programmatic
+// launch, pdl_enter): most of them have little or nothing to do in a tick and
+// would otherwise cost a full launch gap each. The first kernel of a graph has
+// no predecessor to overlap.
+void eng_tick(const EngDev &d, int tpm, const TickExtent &x, bool first, cudaStream_t st)
 {
     const int slots = std::min(x.slots, d.nslots);
     const int gm = sgrid(std::min(x.mols, d.mol_cap), 256, 8);
-    const int gc = sgrid(std::min(x.cells, d.cell_cap), 256, 8);
+    const int gc = sgrid(std::min(x.cells, d.cell_cap), 8, 8);  // a warp per cell
     // the slot loops (decision, all-pairs jobs) stop at the extent: every
     // resident slot lies below it, the ones above are empty
     EngDev dx = d;
     dx.nslots = slots;
-    k_e_decide<<<1, EDEC, 0, st>>>(dx);
-    k_e_wrap_bin<<<gm, 256, 0, st>>>(d);
-    k_e_scan<<<slots, ESCAN, 0, st>>>(d);
-    k_e_scatter<<<gm, 256, 0, st>>>(d);
-    k_e_sort<<<gc, 256, 0, st>>>(d);
-    k_e_reorder_gather<<<gm, 256, 0, st>>>(d);
-    k_e_reorder_copy<<<gm, 256, 0, st>>>(d);
+    pdl_capture = first;
+    pdl_launch(k_e_decide, 1, EDEC, st, dx);
+    pdl_capture = false;
+    pdl_launch(k_e_wrap_bin, gm, 256, st, d);
+    pdl_launch(k_e_scan, slots, ESCAN, st, d);
+    pdl_launch(k_e_scatter, gm, 256, st, d);
+    pdl_launch(k_e_sort, gc, 256, st, d);
+    pdl_launch(k_e_reorder_gather, gm, 256, st, d);
+    pdl_launch(k_e_reorder_copy, gm, 256, st, d);
     // at most one resident wave
-    k_e_build<<<sgrid(std::min(x.cells, d.cell_cap), NB_WARPS, 6), NB_THREADS, 0, st>>>(d);
+    pdl_launch(k_e_build, sgrid(std::max(std::min(x.cells, d.cell_cap), std::min(x.mols, d.mol_cap)), NB_WARPS, 6), NB_THREADS, st, d);
     launch_force_any(d, tpm, std::min(x.mols, d.mol_cap), false, st);
     const dim3 gap(std::min(slots, EAP_XBLOCKS), EAP_YBLOCKS);
-    if (d.precision == 0) k_e_force_ap<0><<<gap, EAP_THREADS, 0, st>>>(dx);
-    else k_e_force_ap<1><<<gap, EAP_THREADS, 0, st>>>(dx);
-    k_e_thermo<<<dim3(slots, EY), ER, 0, st>>>(d);
-    k_e_move_lfv<<<gm, 256, 0, st>>>(d);
-    k_e_record<<<dim3(slots, EY), ER, 0, st>>>(d);
+    if (d.precision == 0) pdl_launch(k_e_force_ap<0>, gap, EAP_THREADS, st, dx);
+    else pdl_launch(k_e_force_ap<1>, gap, EAP_THREADS, st, dx);
+    pdl_launch(k_e_thermo, dim3(slots, EY), ER, st, d);
+    pdl_launch(k_e_move_lfv, gm, 256, st, d);
+    pdl_launch(k_e_record, dim3(slots, EY), ER, st, d);
 }
 
 void eng_build_only(const EngDev &d, int cells, cudaStream_t st)

@@ -30,6 +30,7 @@
 #include <string>
 
 #include "flowmol_b200.h"
+#include "fm_rows.cuh"
 
 namespace {
 
@@ -56,6 +57,10 @@ struct NaGeom {
     int precision;
     int want_pe, want_vir;
 };
+
+// Status word: a molecule outside the grid; a real molecule in a halo cell
+// (a coordinate exactly on a lower face).
+constexpr unsigned NA_ESCAPE = 1u, NA_STRAYS = 2u;
 
 struct NaScratch {
     unsigned int *status;
@@ -105,33 +110,38 @@ __device__ __forceinline__ double na_wrap(double x, double hd, double L)
     return x;
 }
 
-__global__ void k_na_bin(NaGeom g, NaScratch s, const double *r3)
+__device__ __forceinline__ bool halo_axis(int x, int ne) { return x == 0 || x == ne - 1; }
+
+// The wrapped position of molecule i and its cell.
+__device__ __forceinline__ double4 na_place(const NaGeom &g, const NaScratch &s, const double *r3, int i, int &cell)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g.n) return;
     bool bad = false;
     const double x = na_wrap(r3[3 * (size_t)i], g.hd[0], g.L[0]);
     const double y = na_wrap(r3[3 * (size_t)i + 1], g.hd[1], g.L[1]);
     const double z = na_wrap(r3[3 * (size_t)i + 2], g.hd[2], g.L[2]);
-    int cx = na_bin(x, g.hd[0], g.cs[0], g.ne[0], bad);
-    int cy = na_bin(y, g.hd[1], g.cs[1], g.ne[1], bad);
-    int cz = na_bin(z, g.hd[2], g.cs[2], g.ne[2], bad);
-    if (bad) atomicOr(s.status, 1u);
-    int c = cx + g.ne[0] * (cy + g.ne[1] * cz);
+    const int cx = na_bin(x, g.hd[0], g.cs[0], g.ne[0], bad);
+    const int cy = na_bin(y, g.hd[1], g.cs[1], g.ne[1], bad);
+    const int cz = na_bin(z, g.hd[2], g.cs[2], g.ne[2], bad);
+    if (bad) atomicOr(s.status, NA_ESCAPE);
+    if (halo_axis(cx, g.ne[0]) || halo_axis(cy, g.ne[1]) || halo_axis(cz, g.ne[2])) atomicOr(s.status, NA_STRAYS);
+    cell = cx + g.ne[0] * (cy + g.ne[1] * cz);
+    return make_double4(x, y, z, (double)i);
+}
+
+__global__ void k_na_bin(NaGeom g, NaScratch s, const double *r3)
+{
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= g.n) return;
+    int c;
+    na_place(g, s, r3, i, c);
     s.cell_of[i] = c;
     atomicAdd(&s.count[c], 1);
 }
 
-constexpr int NA_SCAN = 1024;
-__global__ void __launch_bounds__(NA_SCAN) k_na_scan(NaGeom g, NaScratch s)
+// Exclusive sum of `local` over the block's 1024 threads.
+__device__ __forceinline__ int na_block_scan(int local, int *ws)
 {
-    __shared__ int ws[32];
-    const int nc = g.ncell;
-    const int per = (nc + NA_SCAN - 1) / NA_SCAN;
-    const int b = threadIdx.x * per, e = min(b + per, nc);
-    int local = 0;
-    for (int c = b; c < e; c++) local += s.count[c];
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int incl = local;
     for (int o = 1; o < 32; o <<= 1) {
         int t = __shfl_up_sync(0xffffffffu, incl, o);
@@ -148,7 +158,64 @@ __global__ void __launch_bounds__(NA_SCAN) k_na_scan(NaGeom g, NaScratch s)
         ws[lane] = vi - v;
     }
     __syncthreads();
-    int run = ws[w] + incl - local;
+    return ws[w] + incl - local;
+}
+
+// Deterministic order of a cell's records [b, e): by original index, by one
+// warp. A lane holds up to NA_HELD records and counts the ones before each;
+// larger cells are sorted by lane 0.
+constexpr int NA_HELD = 4;
+__device__ __forceinline__ void na_sort_cell(double4 *spos, int b, int e, int lane)
+{
+    const int m = e - b;
+    if (m <= 1) return;
+    if (m > 32 * NA_HELD) {
+        if (lane == 0)
+            for (int x = b + 1; x < e; x++) {
+                const double4 key = spos[x];
+                int y = x - 1;
+                while (y >= b && spos[y].w > key.w) {
+                    spos[y + 1] = spos[y];
+                    y--;
+                }
+                spos[y + 1] = key;
+            }
+        return;
+    }
+    double4 p[NA_HELD];
+    int id[NA_HELD], rank[NA_HELD];
+#pragma unroll
+    for (int q = 0; q < NA_HELD; q++) {
+        const bool in = 32 * q + lane < m;
+        p[q] = in ? spos[b + 32 * q + lane] : make_double4(0, 0, 0, 0);
+        id[q] = in ? (int)p[q].w : 0x7fffffff;
+        rank[q] = 0;
+    }
+#pragma unroll
+    for (int k = 0; k < NA_HELD; k++) {
+        if (32 * k >= m) break;
+        for (int l = 0; l < min(32, m - 32 * k); l++) {
+            const int other = __shfl_sync(0xffffffffu, id[k], l);
+#pragma unroll
+            for (int q = 0; q < NA_HELD; q++) rank[q] += other < id[q] ? 1 : 0;
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < NA_HELD; q++)
+        if (32 * q + lane < m) spos[b + rank[q]] = p[q];
+}
+
+constexpr int NA_SCAN = 1024;
+__global__ void __launch_bounds__(NA_SCAN) k_na_scan(NaGeom g, NaScratch s)
+{
+    __shared__ int ws[32];
+    const int nc = g.ncell;
+    const int per = (nc + NA_SCAN - 1) / NA_SCAN;
+    const int b = threadIdx.x * per, e = min(b + per, nc);
+    int local = 0;
+    for (int c = b; c < e; c++) local += s.count[c];
+    int run = na_block_scan(local, ws);
     for (int c = b; c < e; c++) {
         int k = s.count[c];
         s.start[c] = run;
@@ -169,90 +236,150 @@ __global__ void k_na_scatter(NaGeom g, NaScratch s, const double *r3)
                                 na_wrap(r3[3 * (size_t)i + 2], g.hd[2], g.L[2]), (double)i);
 }
 
-// Deterministic in-cell order (by original index).
 __global__ void k_na_sort(NaGeom g, NaScratch s)
 {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= g.ncell) return;
-    int b = s.start[c], e = s.start[c + 1];
-    for (int x = b + 1; x < e; x++) {
-        double4 key = s.spos[x];
-        int y = x - 1;
-        while (y >= b && s.spos[y].w > key.w) {
-            s.spos[y + 1] = s.spos[y];
-            y--;
-        }
-        s.spos[y + 1] = key;
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (c < g.ncell) na_sort_cell(s.spos, s.start[c], s.start[c + 1], threadIdx.x & 31);
+}
+
+// Everything before the forces in one block, the cell counts in shared memory:
+// up to NA_SMALL_N molecules five small kernels would mostly wait for each
+// other's launch.
+constexpr int NA_SMALL_N = 4096, NA_SMALL_CELLS = 8192;
+__global__ void __launch_bounds__(NA_SCAN) k_na_cells(NaGeom g, NaScratch s, const double *r3)
+{
+    __shared__ int ws[32];
+    __shared__ int count[NA_SMALL_CELLS];
+    const int nc = g.ncell;
+    for (int c = threadIdx.x; c < nc; c += NA_SCAN) count[c] = 0;
+    if (threadIdx.x == 0) *s.status = 0u;
+    __syncthreads();
+    double4 p[NA_SMALL_N / NA_SCAN];
+    int cell[NA_SMALL_N / NA_SCAN];
+#pragma unroll
+    for (int q = 0; q < NA_SMALL_N / NA_SCAN; q++) {
+        const int i = q * NA_SCAN + threadIdx.x;
+        if (i >= g.n) break;
+        p[q] = na_place(g, s, r3, i, cell[q]);
+        s.cell_of[i] = cell[q];
+        atomicAdd(&count[cell[q]], 1);
+    }
+    __syncthreads();
+    const int per = (nc + NA_SCAN - 1) / NA_SCAN;
+    const int b = min((int)threadIdx.x * per, nc), e = min(b + per, nc);
+    int local = 0;
+    for (int c = b; c < e; c++) local += count[c];
+    int run = na_block_scan(local, ws);
+    for (int c = b; c < e; c++) {
+        const int k = count[c];
+        s.start[c] = run;
+        count[c] = run;  // from here on the cell's next free place
+        run += k;
+    }
+    if (threadIdx.x == NA_SCAN - 1) s.start[nc] = run;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NA_SMALL_N / NA_SCAN; q++) {
+        if (q * NA_SCAN + (int)threadIdx.x >= g.n) break;
+        s.spos[atomicAdd(&count[cell[q]], 1)] = p[q];
+    }
+    __syncthreads();
+    for (int c = threadIdx.x >> 5; c < nc; c += NA_SCAN / 32)
+        na_sort_cell(s.spos, s.start[c], s.start[c + 1], threadIdx.x & 31);
+}
+
+// One pair: forces, energy and virial (LJ_accijmag, LJ_energy).
+template <int PREC>
+__device__ __forceinline__ void na_pair(double r2, double dx, double dy, double dz, double potshift, double (&f)[5])
+{
+    if (PREC == 0) {
+        const double sv = 1.0 / r2, s2 = sv * sv, s4 = s2 * s2;
+        const double acc = 48.0 * (s4 * s2 * sv - 0.5 * s4);
+        f[0] += acc * dx; f[1] += acc * dy; f[2] += acc * dz;
+        const double s3 = s2 * sv;
+        f[3] += 4.0 * (s3 * s3 - s3) - potshift;
+        f[4] += acc * r2;
+    } else {
+        // the precision form of the main force kernel: FP32 pair
+        // magnitude, scaled by the FP64 rij, sums in FP64
+        const float sv = __frcp_rn((float)r2), s2 = sv * sv, s4 = s2 * s2;
+        const double acc = (double)(48.0f * (s4 * s2 * sv - 0.5f * s4));
+        f[0] = fma(acc, dx, f[0]); f[1] = fma(acc, dy, f[1]); f[2] = fma(acc, dz, f[2]);
+        const float s3 = s2 * sv, s6 = s3 * s3;
+        f[3] += (double)(4.0f * (s6 - s3)) - potshift;
+        f[4] += acc * r2;
     }
 }
 
-__device__ __forceinline__ bool halo_axis(int x, int ne) { return x == 0 || x == ne - 1; }
-
-// One thread per molecule (cell order): every candidate of the 27 cells
-// around its cell that are not both halo with it -- real molecules of the
-// cell, plus, for a halo cell, the images of the interior cell on the far
-// side shifted by +/-domain -- tested against rcutoff2 in FP64.
-template <int PREC>
-__global__ void k_na_force(NaGeom g, NaScratch s, double *a3, double *pe_out, double *vir_out)
+// G lanes per molecule (cell order) over the candidate ranges of the list build
+// (rows_range, rows_strays): the molecules of the 27 cells around its cell that
+// are not both halo with it, and for a halo cell the images of the interior
+// cell on the far side, tested against rcutoff2 in FP64. The lanes' sums meet
+// in a fixed tree. One lane per molecule, cell by cell, was a chain of some
+// 500 dependent tests: 200 us for 1,008 molecules.
+template <int PREC, int G>
+__global__ void __launch_bounds__(fm::ROWS_THREADS) k_na_force(NaGeom g, NaScratch s, double *a3, double *pe_out, double *vir_out)
 {
-    int slot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot >= g.n) return;
-    const double4 pi = s.spos[slot];
-    const int i = (int)pi.w;
-    const int c = s.cell_of[i];
-    const int cx = c % g.ne[0], cy = (c / g.ne[0]) % g.ne[1], cz = c / (g.ne[0] * g.ne[1]);
-    const bool chalo = halo_axis(cx, g.ne[0]) || halo_axis(cy, g.ne[1]) || halo_axis(cz, g.ne[2]);
-    double fx = 0.0, fy = 0.0, fz = 0.0, pe = 0.0, vir = 0.0;
-    for (int q = 0; q < 27; q++) {
-        int x2 = cx + q % 3 - 1, y2 = cy + (q / 3) % 3 - 1, z2 = cz + q / 9 - 1;
-        if (x2 < 0 || y2 < 0 || z2 < 0 || x2 >= g.ne[0] || y2 >= g.ne[1] || z2 >= g.ne[2]) continue;
-        bool h2 = halo_axis(x2, g.ne[0]) || halo_axis(y2, g.ne[1]) || halo_axis(z2, g.ne[2]);
-        if (chalo && h2) continue;
-        for (int pass = 0; pass < (h2 ? 2 : 1); pass++) {
-            int sx = 0, sy = 0, sz = 0, src = x2 + g.ne[0] * (y2 + g.ne[1] * z2);
-            if (pass == 1) {
-                sx = x2 == 0 ? -1 : (x2 == g.ne[0] - 1 ? 1 : 0);
-                sy = y2 == 0 ? -1 : (y2 == g.ne[1] - 1 ? 1 : 0);
-                sz = z2 == 0 ? -1 : (z2 == g.ne[2] - 1 ? 1 : 0);
-                int xs = x2 == 0 ? g.ne[0] - 2 : (x2 == g.ne[0] - 1 ? 1 : x2);
-                int ys = y2 == 0 ? g.ne[1] - 2 : (y2 == g.ne[1] - 1 ? 1 : y2);
-                int zs = z2 == 0 ? g.ne[2] - 2 : (z2 == g.ne[2] - 1 ? 1 : z2);
-                src = xs + g.ne[0] * (ys + g.ne[1] * zs);
+    __shared__ fm::RowsShared<G> shw[fm::ROWS_THREADS / 32];
+    fm::RowsShared<G> &sh = shw[threadIdx.x >> 5];
+    const int slot = (int)(((long long)blockIdx.x * fm::ROWS_THREADS + threadIdx.x) / G), lane = threadIdx.x % G;
+    const bool on = slot < g.n;
+    double f[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    int i = 0;
+    if (on) {
+        const double4 pi = s.spos[slot];
+        i = (int)pi.w;
+        const int c = s.cell_of[i];
+        const int cx = c % g.ne[0], cy = (c / g.ne[0]) % g.ne[1], cz = c / (g.ne[0] * g.ne[1]);
+        fm::CellSys y;
+        y.cell_start = s.start;
+        y.mol_off = 0;
+        y.dd = 0;
+        for (int k = 0; k < 3; k++) y.ne[k] = g.ne[k];
+        const int self = slot | (fm::NB_NOSHIFT << fm::NB_SHIFT_BITS);
+        auto range = [&](int b, int e, int code) {
+            const int im = code >> fm::NB_SHIFT_BITS;
+            for (int j = b + lane; j < e; j += G) {
+                const double4 pj = fm::ldg_pos(s.spos + j);
+                const double xj = fm::image(pj.x, (im & 3) - 1, g.L[0]);
+                const double yj = fm::image(pj.y, ((im >> 2) & 3) - 1, g.L[1]);
+                const double zj = fm::image(pj.z, ((im >> 4) & 3) - 1, g.L[2]);
+                const double dx = __dsub_rn(pi.x, xj), dy = __dsub_rn(pi.y, yj), dz = __dsub_rn(pi.z, zj);
+                const double r2 = n2(dx, dy, dz);
+                if (r2 < g.rc2 && (j | code) != self) na_pair<PREC>(r2, dx, dy, dz, g.potshift, f);
             }
-            const int b = s.start[src], e = s.start[src + 1];
-            for (int j = b; j < e; j++) {
-                if (j == slot && pass == 0) continue;
-                double4 pj = s.spos[j];
-                double xj = sx ? __dadd_rn(pj.x, sx > 0 ? g.L[0] : -g.L[0]) : pj.x;
-                double yj = sy ? __dadd_rn(pj.y, sy > 0 ? g.L[1] : -g.L[1]) : pj.y;
-                double zj = sz ? __dadd_rn(pj.z, sz > 0 ? g.L[2] : -g.L[2]) : pj.z;
-                double dx = __dsub_rn(pi.x, xj), dy = __dsub_rn(pi.y, yj), dz = __dsub_rn(pi.z, zj);
-                double r2 = n2(dx, dy, dz);
-                if (r2 < g.rc2) {
-                    if (PREC == 0) {
-                        const double sv = 1.0 / r2, s2 = sv * sv, s4 = s2 * s2;
-                        const double acc = 48.0 * (s4 * s2 * sv - 0.5 * s4);
-                        fx += acc * dx; fy += acc * dy; fz += acc * dz;
-                        const double s3 = s2 * sv;
-                        pe += 4.0 * (s3 * s3 - s3) - g.potshift;
-                        vir += acc * r2;
-                    } else {
-                        // the precision form of the main force kernel: FP32 pair
-                        // magnitude, scaled by the FP64 rij, sums in FP64
-                        const float sv = __frcp_rn((float)r2), s2 = sv * sv, s4 = s2 * s2;
-                        const double acc = (double)(48.0f * (s4 * s2 * sv - 0.5f * s4));
-                        fx = fma(acc, dx, fx); fy = fma(acc, dy, fy); fz = fma(acc, dz, fz);
-                        const float s3 = s2 * sv, s6 = s3 * s3;
-                        pe += (double)(4.0f * (s6 - s3)) - g.potshift;
-                        vir += acc * r2;
-                    }
-                }
+        };
+        if (*s.status & NA_STRAYS) {
+            fm::rows_strays(y, cx, cy, cz, range);
+        } else if (!(*s.status & NA_ESCAPE)) {
+            const unsigned group = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(G - 1));
+            const int n = fm::rows_count(y, cx), gi = (threadIdx.x & 31) / G;
+            for (int r = lane; r < n; r += G) {
+                int b, e, code;
+                fm::rows_range(y, cx, cy, cz, n, r, b, e, code);
+                sh.be[gi][r] = make_int2(b, e);
+                sh.code[gi][r] = code;
             }
+            __syncwarp(group);
+            for (int r = 0; r < n; r++) range(sh.be[gi][r].x, sh.be[gi][r].y, sh.code[gi][r]);
         }
     }
-    a3[3 * (size_t)i] = fx; a3[3 * (size_t)i + 1] = fy; a3[3 * (size_t)i + 2] = fz;
-    if (pe_out) pe_out[i] = pe;
-    if (vir_out) vir_out[i] = vir;
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 5; k++) f[k] += __shfl_xor_sync(0xffffffffu, f[k], o);
+    if (!on || lane != 0) return;
+    a3[3 * (size_t)i] = f[0]; a3[3 * (size_t)i + 1] = f[1]; a3[3 * (size_t)i + 2] = f[2];
+    if (pe_out) pe_out[i] = f[3];
+    if (vir_out) vir_out[i] = f[4];
+}
+
+template <int G>
+void na_force(const NaGeom &g, const NaScratch &s, double *a, double *pe, double *vir, cudaStream_t st)
+{
+    const int blocks = (int)(((long long)g.n * G + fm::ROWS_THREADS - 1) / fm::ROWS_THREADS);
+    if (g.precision == 0) k_na_force<0, G><<<blocks, fm::ROWS_THREADS, 0, st>>>(g, s, a, pe, vir);
+    else k_na_force<1, G><<<blocks, fm::ROWS_THREADS, 0, st>>>(g, s, a, pe, vir);
 }
 
 thread_local std::string g_na_error;
@@ -335,21 +462,26 @@ extern "C" int fm_compute_forces_noalloc(const fm_params *p, int32_t n, const do
     NaScratch s = carve(base);
     cudaStream_t st = (cudaStream_t)cuda_stream;
     const int T = 256;
-    k_na_zero<<<(g.ncell + T - 1) / T, T, 0, st>>>(g, s);
-    k_na_bin<<<(n + T - 1) / T, T, 0, st>>>(g, s, d_r);
-    k_na_scan<<<1, NA_SCAN, 0, st>>>(g, s);
-    k_na_scatter<<<(n + T - 1) / T, T, 0, st>>>(g, s, d_r);
-    k_na_sort<<<(g.ncell + 127) / 128, 128, 0, st>>>(g, s);
-    if (g.precision == 0)
-        k_na_force<0><<<(n + 127) / 128, 128, 0, st>>>(g, s, d_a, d_potenergymol, d_virialmol);
-    else
-        k_na_force<1><<<(n + 127) / 128, 128, 0, st>>>(g, s, d_a, d_potenergymol, d_virialmol);
+    if (n <= NA_SMALL_N && g.ncell <= NA_SMALL_CELLS) {
+        k_na_cells<<<1, NA_SCAN, 0, st>>>(g, s, d_r);
+    } else {
+        k_na_zero<<<(g.ncell + T - 1) / T, T, 0, st>>>(g, s);
+        k_na_bin<<<(n + T - 1) / T, T, 0, st>>>(g, s, d_r);
+        k_na_scan<<<1, NA_SCAN, 0, st>>>(g, s);
+        k_na_scatter<<<(n + T - 1) / T, T, 0, st>>>(g, s, d_r);
+        k_na_sort<<<(g.ncell + 3) / 4, 128, 0, st>>>(g, s);
+    }
+    switch (fm::rows_lanes((double)n / (g.L[0] * g.L[1] * g.L[2]) * g.cs[0] * g.cs[1] * g.cs[2])) {
+    case 8: na_force<8>(g, s, d_a, d_potenergymol, d_virialmol, st); break;
+    case 16: na_force<16>(g, s, d_a, d_potenergymol, d_virialmol, st); break;
+    default: na_force<32>(g, s, d_a, d_potenergymol, d_virialmol, st); break;
+    }
     e = cudaGetLastError();
     if (e != cudaSuccess) return na_fail(FM_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     unsigned int status = 0;
     e = cudaMemcpyAsync(&status, s.status, sizeof status, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return na_fail(FM_ERR_CUDA, std::string("status read: ") + cudaGetErrorString(e));
-    if (status & 1u) return na_fail(FM_ERR_ESCAPE, "a molecule lies outside the cell grid");
+    if (status & NA_ESCAPE) return na_fail(FM_ERR_ESCAPE, "a molecule lies outside the cell grid");
     return FM_OK;
 }

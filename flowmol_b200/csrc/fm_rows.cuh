@@ -21,11 +21,10 @@
 // molecule is short, where the build by warp (fm_build.cuh: a cell, or 2x2x2 of
 // them, per warp) waits for the serial work of one warp, ~100 us however small
 // the system is: a rebuild of 2,048 LJ molecules costs 34 us instead of 132,
-// one of 32,000 104 instead of 152, a Soddemann solution of 25,092 beads (bonds
-// looked up as well) 58 us for the rows instead of 290. Bound by issue at
-// larger sizes (~45 instructions a step beside the 8 FP64 ones): at 108,000
-// molecules 264 us against 160 by warp, whose shared staging tests four owners
-// per candidate loaded.
+// one of 32,000 90 instead of 152 (by fours, below). Bound by issue at larger
+// sizes (some 80 instructions a step, 8 of them FP64): at 108,000 molecules 170
+// us by fours and 264 by molecule against 160 by warp, whose staging in shared
+// memory tests four owners per candidate loaded.
 #pragma once
 #include "fm_build.cuh"
 
@@ -92,18 +91,18 @@ __device__ __forceinline__ void rows_strays(const CellSys &y, int cx, int cy, in
     }
 }
 
-// A group's ranges, worked out one per lane.
+// The ranges of a warp's groups, worked out one per lane.
 template <int G>
 struct RowsShared {
-    int2 be[ROWS_THREADS / G][18];
-    int code[ROWS_THREADS / G][18];
+    int2 be[32 / G][18];
+    int code[32 / G][18];
 };
 
 // Row of molecule i (cell c) of system y by the G consecutive lanes of a warp
-// that are given it (lane g of them). Returns the row's length and, through
-// nb, its number of bonds, to every lane of the group.
-template <int G, bool POLY>
-__device__ __forceinline__ int rows_build(const CellSys &y, int i, int c, bool strays, int g, RowsShared<G> &sh, int &nb)
+// that are given it (lane g of them). Returns the row's length to every lane of
+// the group.
+template <int G>
+__device__ __forceinline__ int rows_build(const CellSys &y, int i, int c, bool strays, int g, RowsShared<G> &sh)
 {
     const unsigned shift = (threadIdx.x & 31u) & ~(unsigned)(G - 1);
     const unsigned ones = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
@@ -112,10 +111,6 @@ __device__ __forceinline__ int rows_build(const CellSys &y, int i, int c, bool s
     const int maxn = y.maxn;
     int32_t *const row = y.nbr + nb_row(i, maxn);
     int cnt = 0;
-    nb = 0;
-    int4 bf = make_int4(0, 0, 0, 0);
-    int ochain = 0;
-    if (POLY) { ochain = y.chain[i]; bf = y.bflag[i]; }
     const int cx = c % y.ne[0], cy = (c / y.ne[0]) % y.ne[1], cz = c / (y.ne[0] * y.ne[1]);
     const int self_e = i | (NB_NOSHIFT << NB_SHIFT_BITS);
     auto scan = [&](int b, int e, int code) {
@@ -136,25 +131,13 @@ __device__ __forceinline__ int rows_build(const CellSys &y, int i, int c, bool s
             const int at = cnt + __popc(m & lt);
             if (hit && at < maxn) row[nb_col(at)] = j | code;
             cnt += __popc(m);
-            if (POLY) {  // a candidate of the owner's chain whose subchain bit is set is bonded
-                bool bond = in && y.chain[in ? j : b] == ochain && (j | code) != self_e;
-                if (__any_sync(group, bond)) {
-                    const int pos = bond ? y.subchain[j] - 1 : -1, grp = pos / 31;
-                    const int word = grp == 0 ? bf.x : grp == 1 ? bf.y : grp == 2 ? bf.z : bf.w;
-                    bond = pos >= 0 && grp < 4 && ((word >> (pos % 31)) & 1);
-                    const unsigned mb = (__ballot_sync(group, bond) >> shift) & ones;
-                    const int bat = nb + __popc(mb & lt);
-                    if (bond && bat < 4) y.bnd[(size_t)i * 4 + bat] = j | code;
-                    nb += __popc(mb);
-                }
-            }
         }
     };
     if (strays) {
         rows_strays(y, cx, cy, cz, scan);
         return cnt;
     }
-    const int n = rows_count(y, cx), gi = threadIdx.x / G;
+    const int n = rows_count(y, cx), gi = (threadIdx.x & 31) / G;
     __syncwarp(group);
     for (int r = g; r < n; r += G) {
         int b, e, code;
@@ -169,6 +152,114 @@ __device__ __forceinline__ int rows_build(const CellSys &y, int i, int c, bool s
         scan(be.x, be.y, sh.code[gi][r]);
     }
     return cnt;
+}
+
+// Rows of up to four molecules i0 .. i0 + own - 1 of cell c by a warp: as
+// rows_build with 32 lanes, the four tests of a candidate sharing its load and
+// the walk over the ranges (80 -> 45 instructions a test). Returns the longest
+// row.
+__device__ __forceinline__ int rows_four(const CellSys &y, int i0, int own, int n, bool strays, int cx, int cy, int cz,
+                                         int lane, RowsShared<32> &sh)
+{
+    const unsigned lt = (1u << lane) - 1u;
+    const int maxn = y.maxn;
+    double ox[4], oy[4], oz[4];
+    int cnt[4];
+    unsigned row[4];
+    int32_t *const base = y.nbr + nb_row(i0, maxn);  // the four rows are within one group's width of it
+#pragma unroll
+    for (int w = 0; w < 4; w++) {
+        const int i = i0 + min(w, own - 1);
+        const double4 p = ldg_pos(y.P + i);
+        ox[w] = w < own ? p.x : 1e30; oy[w] = p.y; oz[w] = p.z;  // no molecule: r^2 is huge
+        row[w] = (unsigned)(nb_row(i, maxn) - nb_row(i0, maxn));
+        cnt[w] = 0;
+    }
+    auto scan = [&](int b, int e, int code) {
+        const bool shifted = code != NB_NOSHIFT << NB_SHIFT_BITS;
+        for (int k = b; k < e; k += 32) {
+            const int j = k + lane;
+            const double4 p = ldg_pos(y.P + min(j, e - 1));
+            double xj = p.x, yj = p.y, zj = p.z;
+            if (shifted) {
+                const int im = code >> NB_SHIFT_BITS;
+                xj = image(xj, (im & 3) - 1, y.L[0]);
+                yj = image(yj, ((im >> 2) & 3) - 1, y.L[1]);
+                zj = image(zj, ((im >> 4) & 3) - 1, y.L[2]);
+            }
+            if (j >= e) xj = -1e30;
+            const int self = shifted ? -1 : j - i0;  // 0 .. 3: the candidate is that molecule
+#pragma unroll
+            for (int w = 0; w < 4; w++) {
+                const double r2 = norm2_rn(__dsub_rn(ox[w], xj), __dsub_rn(oy[w], yj), __dsub_rn(oz[w], zj));
+                const bool hit = r2 < y.rn2 && self != w;
+                const unsigned m = __ballot_sync(0xffffffffu, hit);
+                const int at = cnt[w] + __popc(m & lt);
+                if (hit && at < maxn) base[row[w] + (unsigned)nb_col(at)] = j | code;
+                cnt[w] += __popc(m);
+            }
+        }
+    };
+    if (strays) {
+        rows_strays(y, cx, cy, cz, scan);
+    } else {
+#pragma unroll 1
+        for (int r = 0; r < n; r++) scan(sh.be[0][r].x, sh.be[0][r].y, sh.code[0][r]);
+    }
+    int most = 0;
+#pragma unroll
+    for (int w = 0; w < 4; w++) {
+        if (lane == w && w < own) y.nnbr[i0 + w] = min(cnt[w], maxn);
+        most = max(most, cnt[w]);
+    }
+    return most;
+}
+
+// Unit u of the build by fours: ROWS_SPLIT warps share an interior cell. Where
+// halo cells have molecules (strays, or a subdomain's copies, which get no
+// rows), the first of a cell's warps looks after an equal share of them.
+constexpr int ROWS_SPLIT = 5;
+constexpr int ROWS_FOUR_MOLECULES = 16384;  // a warp's chain is longer: 2,048 molecules 50 us a rebuild against 34
+__host__ __device__ inline int rows_four_units(const int (&ne)[3])
+{
+    return (ne[0] - 2) * (ne[1] - 2) * (ne[2] - 2) * ROWS_SPLIT;
+}
+__device__ __forceinline__ int rows_four_unit(const CellSys &y, int u, bool strays, int lane, RowsShared<32> &sh)
+{
+    const int ne0 = y.ne[0], ne1 = y.ne[1], ne2 = y.ne[2];
+    const int q = u / ROWS_SPLIT, part = u % ROWS_SPLIT;
+    const int cx = 1 + q % (ne0 - 2), cy = 1 + (q / (ne0 - 2)) % (ne1 - 2), cz = 1 + q / ((ne0 - 2) * (ne1 - 2));
+    const int c = cx + ne0 * (cy + ne1 * cz);
+    int most = 0;
+    const int b = y.cell_start[c] - y.mol_off, m = y.cell_start[c + 1] - y.mol_off - b;
+    if (4 * part < m) {
+        const int n = rows_count(y, cx);
+        __syncwarp();
+        if (!strays && lane < n) {
+            int rb, re, code;
+            rows_range(y, cx, cy, cz, n, lane, rb, re, code);
+            sh.be[0][lane] = make_int2(rb, re);
+            sh.code[0][lane] = code;
+        }
+        __syncwarp();
+        for (int g = 4 * part; g < m; g += 4 * ROWS_SPLIT)
+            most = max(most, rows_four(y, b + g, min(4, m - g), n, strays, cx, cy, cz, lane, sh));
+    }
+    if ((strays || y.dd) && part == 0) {
+        const int nint = (ne0 - 2) * (ne1 - 2) * (ne2 - 2);
+        for (int h = q; h < ne0 * ne1 * ne2; h += nint) {
+            const int hx = h % ne0, hy = (h / ne0) % ne1, hz = h / (ne0 * ne1);
+            if (!(is_halo(hx, ne0) || is_halo(hy, ne1) || is_halo(hz, ne2))) continue;
+            const int hb = y.cell_start[h] - y.mol_off, hm = y.cell_start[h + 1] - y.mol_off - hb;
+            if (y.dd) {
+                for (int k = lane; k < hm; k += 32) y.nnbr[hb + k] = 0;
+                continue;
+            }
+            for (int g = 0; g < hm; g += 4)
+                most = max(most, rows_four(y, hb + g, min(4, hm - g), 0, true, hx, hy, hz, lane, sh));
+        }
+    }
+    return most;
 }
 
 }  // namespace fm
