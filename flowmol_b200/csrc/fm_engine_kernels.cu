@@ -604,7 +604,7 @@ constexpr int EF_THREADS = 256;
 // record this tick (forces only: few registers, full occupancy), REC true the
 // recording ones (PE, virial and the pressure-tensor terms as well).
 template <int TPM, int PREC, bool FORCE_ONLY, bool REC>
-__global__ void __launch_bounds__(EF_THREADS, REC ? 2 : 4) k_e_force(EngDev d)
+__global__ void __launch_bounds__(EF_THREADS, 4) k_e_force(EngDev d)
 {
     pdl_enter();
     constexpr int PER_BLOCK = EF_THREADS / TPM;

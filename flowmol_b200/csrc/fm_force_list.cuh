@@ -218,11 +218,13 @@ __device__ __forceinline__ double owner_finish(const FmDev &d, int pset, const d
 }
 
 // Four resident blocks hide the gathers' latency (three, at 66 registers,
-// take 0.31 ms instead of 0.27 at 1M); record steps carry more sums.  Lanes on
+// take 0.31 ms instead of 0.27 at 1M), on record steps too, although their sums
+// spill a little: 0.48 -> 0.40 ms at 1M in FP64, 77 -> 63 us at 108,000 with the
+// pressure tensor, against two blocks.  Lanes on
 // neighbouring entries against lanes on four entries each: 338 -> 308 us with
 // four lanes at 1M, 42.4 -> 36.7 at 108,000, 19.6 -> 17.7 at 32,000.
 template <int TPM, bool REC, int MODE, int PREC>
-__global__ void __launch_bounds__(FORCE_THREADS, REC || (PREC & 6) != 0 ? 2 : 4) k_force(FmDev d)
+__global__ void __launch_bounds__(FORCE_THREADS, (PREC & 6) != 0 ? 2 : 4) k_force(FmDev d)
 {
     pdl_enter();
     if (frozen(d)) return;
