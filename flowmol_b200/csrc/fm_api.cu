@@ -558,8 +558,15 @@ static int begin_state(fm_handle *h, int32_t n)
 static int set_glob(fm_handle *h, const int32_t *glob_no)
 {
     const int n = h->d.n;
-    h->glob_host.resize((size_t)n);
-    for (int i = 0; i < n; i++) h->glob_host[(size_t)i] = glob_no ? glob_no[i] : i + 1;
+    if (!glob_no) {
+        // numbered as uploaded: the device writes it, the host copy is fetched
+        // when something asks for it (filled here and copied over, 1M numbers
+        // took 1.5 ms of every upload)
+        h->glob_host.clear();
+        fm::launch_count_up(h->glob, n, h->st);
+        return FM_OK;
+    }
+    h->glob_host.assign(glob_no, glob_no + n);
     FM_CUDA(cudaMemcpyAsync(h->glob, h->glob_host.data(), sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, h->st));
     return FM_OK;
 }
@@ -718,6 +725,8 @@ extern "C" int fm_set_mie(fm_handle *h, const fm_mie_tables *t, const int32_t *m
 }
 
 
+static int pull_glob(fm_handle *h);
+
 extern "C" int fm_get_bonds(fm_handle *h, int32_t *owner, int32_t *partner, int8_t *code, int64_t cap, int64_t *n_out)
 {
     FM_TRY(ready(h, 2));
@@ -729,6 +738,7 @@ extern "C" int fm_get_bonds(fm_handle *h, int32_t *owner, int32_t *partner, int8
     FM_CUDA(cudaMemcpyAsync(slot.data(), h->d.slot_of, 4 * n, cudaMemcpyDeviceToHost, h->st));
     FM_CUDA(cudaMemcpyAsync(bnd.data(), h->d.bnd, 16 * n, cudaMemcpyDeviceToHost, h->st));
     FM_CUDA(cudaStreamSynchronize(h->st));
+    FM_TRY(pull_glob(h));
     int64_t k = 0;
     for (size_t i = 0; i < n; i++)
         for (int b = 0; b < nb[i]; b++) {
@@ -746,11 +756,14 @@ extern "C" int fm_get_bonds(fm_handle *h, int32_t *owner, int32_t *partner, int8
     return FM_OK;
 }
 
-// Global numbers by upload index: once a sort was configured they are
-// renumbered on the device, and the host copy is refreshed before each use.
+// Global numbers by upload index on the host: fetched on first use where the
+// device wrote them, and before each use once a sort was configured, which
+// renumbers them on the device.
 static int pull_glob(fm_handle *h)
 {
-    if (!h->glob_moved || h->glob_host.empty()) return FM_OK;
+    const size_t n = (size_t)h->d.n;
+    if (!h->glob_moved && h->glob_host.size() == n) return FM_OK;
+    h->glob_host.resize(n);
     FM_CUDA(cudaMemcpyAsync(h->glob_host.data(), h->glob, sizeof(int32_t) * h->glob_host.size(),
                             cudaMemcpyDeviceToHost, h->st));
     FM_CUDA(cudaStreamSynchronize(h->st));
@@ -1627,13 +1640,16 @@ extern "C" int fm_get_records(fm_handle *h, fm_macro *out, int32_t cap, int32_t 
     int pending = s.nrec_pending;
     int avail = std::min(pending, rc_cap);
     int take = std::min(avail, cap > 0 ? cap : 0);
-    std::vector<fm::FmRecord> rows((size_t)rc_cap);
-    if (take > 0) {
-        FM_CUDA(cudaMemcpyAsync(rows.data(), h->d.rec, sizeof(fm::FmRecord) * (size_t)rc_cap, cudaMemcpyDeviceToHost,
+    std::vector<fm::FmRecord> rows((size_t)take);
+    if (take > 0) {  // the rows asked for: from the oldest to the ring's end, then from its start
+        const int oldest = (pending - avail) % rc_cap, tail = std::min(take, rc_cap - oldest);
+        FM_CUDA(cudaMemcpyAsync(rows.data(), h->d.rec + oldest, sizeof(fm::FmRecord) * (size_t)tail, cudaMemcpyDeviceToHost,
                                 h->st));
+        if (take > tail)
+            FM_CUDA(cudaMemcpyAsync(rows.data() + tail, h->d.rec, sizeof(fm::FmRecord) * (size_t)(take - tail),
+                                    cudaMemcpyDeviceToHost, h->st));
         FM_CUDA(cudaStreamSynchronize(h->st));
-        int oldest = pending - avail;
-        for (int k = 0; k < take; k++) std::memcpy(&out[k], &rows[(size_t)((oldest + k) % rc_cap)], sizeof(fm_macro));
+        for (int k = 0; k < take; k++) std::memcpy(&out[k], &rows[(size_t)k], sizeof(fm_macro));
     }
     int zero = 0;
     FM_CUDA(cudaMemcpyAsync(&h->d.sc->nrec_pending, &zero, sizeof zero, cudaMemcpyHostToDevice, h->st));

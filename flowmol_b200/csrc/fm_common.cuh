@@ -302,6 +302,7 @@ int all_pairs_blocks(int n);
 // the device layout; `order` maps upload index -> slot.
 void launch_set_types(const FmDev &d, cudaStream_t st);
 void launch_set_bead_flags(const FmDev &d, cudaStream_t st);
+void launch_count_up(int32_t *out, int n, cudaStream_t st);  // 1 .. n
 void launch_scatter_state(const FmDev &d, const double *r3, const double *v3, const double *a3,
                           cudaStream_t st);
 void launch_gather_state(const FmDev &d, double *r3, double *v3, double *a3, int32_t *gid,

@@ -1299,6 +1299,13 @@ void launch_set_types(const FmDev &d, cudaStream_t st) { k_set_w<<<nblk(d.n, 256
 
 void launch_set_bead_flags(const FmDev &d, cudaStream_t st) { k_set_w<<<nblk(d.n, 256), 256, 0, st>>>(d); }
 
+__global__ static void k_count_up(int32_t *out, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = i + 1;
+}
+void launch_count_up(int32_t *out, int n, cudaStream_t st) { k_count_up<<<nblk(n, 256), 256, 0, st>>>(out, n); }
+
 void launch_scatter_state(const FmDev &d, const double *r3, const double *v3, const double *a3, cudaStream_t st)
 {
     k_scatter_state<<<nblk(d.n, 256), 256, 0, st>>>(d, r3, v3, a3);

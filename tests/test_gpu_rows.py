@@ -92,3 +92,27 @@ def test_lanes_of_the_force_kernel_read_every_entry_once(gpu_lib, tpm, precision
     assert n.min() <= 6 and n.max() > 64
     for x, y in zip(*out):
         assert np.abs(x - y).max() <= 1.4e-11
+
+
+def test_numbers_and_records_after_a_device_upload(gpu_lib):
+    """Global numbers of a state uploaded without any are 1 .. n, before and
+    after a sort renumbers them; records come in order across the ring's end."""
+    import ctypes as C
+    import torch
+    r, v, dom = lattice.lj_fluid([6, 6, 6], 0.8, 1.0, 87)
+    r = lattice.jitter(r, 0.04, 88, dom)
+    s = api.MDSystem(api.make_params(len(r), dom, WCA_RC, density=0.8, tplot=1))
+    d = [torch.tensor(x, device="cuda") for x in (r, v)]
+    api.check(gpu_lib.fm_upload_state_device(s.h, len(r), *[C.c_void_p(x.data_ptr()) for x in d]))
+    assert np.array_equal(s.download()[3], np.arange(1, len(r) + 1))
+    s.set_sort(1, 1, 1)
+    s.setup()
+    s.simulation_md(5)
+    assert np.array_equal(np.sort(s.download()[3]), np.arange(1, len(r) + 1))
+    assert [x["iter"] for x in s.records()] == list(range(6))
+    s.simulation_md(4094)
+    first = s.records(7)
+    assert [x["iter"] for x in first] == list(range(6, 13))
+    s.simulation_md(4)
+    assert [x["iter"] for x in s.records()] == list(range(4100, 4104))
+    s.close()
