@@ -630,29 +630,68 @@ __global__ void __launch_bounds__(EF_THREADS, 4) k_e_force(EngDev d)
             const int cnt = d.nnbr[i];
             const int32_t *L = d.nbr + s.list_off + nb_row(i - s.mol_off, s.maxn);
             const double4 *Pj = P + s.mol_off;
-            for (int st = 0; row_first<TPM>(st) < cnt; st++) {
-                const int left = row_left<TPM>(st, lane, cnt);
-                const int4 e4 = row_entries<TPM>(L, st, lane, left);
-                const int ev[4] = {e4.x, e4.y, e4.z, e4.w};
-                double4 pj[4];
+            if constexpr (TPM == 1) {
+                // A lane that has the row to itself reads a whole chunk and takes
+                // its entries in row order, four at a time.  By halves of a chunk
+                // (entries h, h + 4, h + 1, h + 5) the entries that count are no
+                // prefix of the four: four conditions of their own and a step more
+                // for rows that leave 3 or 4 of a chunk, 0.50 ms a tick of 2.0M LJ
+                // molecules against 0.47.
+                for (int k0 = 0; k0 < cnt; k0 += 8) {
+                    const int4 *ch = reinterpret_cast<const int4 *>(L + (size_t)k0 * 32u);
+                    const int4 ea = ld_stream_int4(ch), eb = ld_stream_int4(ch + 1);
+#pragma unroll 1
+                    for (int h = 0; h < 2; h++) {
+                        const int n = cnt - k0 - 4 * h;
+                        if (n <= 0) break;
+                        const int ev[4] = {h ? ea.y : ea.x, h ? ea.w : ea.z, h ? eb.y : eb.x, h ? eb.w : eb.z};
+                        double4 pj[4];
 #pragma unroll
-                for (int q = 0; q < 4; q++)
-                    if (left > row_off<TPM>(q)) pj[q] = ldg_pos(Pj + (ev[q] & NB_INDEX_MASK));
+                        for (int q = 0; q < 4; q++)
+                            if (q < n) pj[q] = ldg_pos(Pj + (ev[q] & NB_INDEX_MASK));
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    if (left <= row_off<TPM>(q)) continue;
-                    const int code = ev[q] >> NB_SHIFT_BITS;
-                    double xj = pj[q].x, yj = pj[q].y, zj = pj[q].z;
-                    if (code != NB_NOSHIFT) {  // rows of boundary cells only
-                        xj = image(xj, (code & 3) - 1, s.L[0]);
-                        yj = image(yj, ((code >> 2) & 3) - 1, s.L[1]);
-                        zj = image(zj, ((code >> 4) & 3) - 1, s.L[2]);
+                        for (int q = 0; q < 4; q++) {
+                            if (q >= n) break;
+                            const int code = ev[q] >> NB_SHIFT_BITS;
+                            double xj = pj[q].x, yj = pj[q].y, zj = pj[q].z;
+                            if (code != NB_NOSHIFT) {  // rows of boundary cells only
+                                xj = image(xj, (code & 3) - 1, s.L[0]);
+                                yj = image(yj, ((code >> 2) & 3) - 1, s.L[1]);
+                                zj = image(zj, ((code >> 4) & 3) - 1, s.L[2]);
+                            }
+                            const double dx = __dsub_rn(pi.x, xj);
+                            const double dy = __dsub_rn(pi.y, yj);
+                            const double dz = __dsub_rn(pi.z, zj);
+                            const double r2 = norm2_rn(dx, dy, dz);
+                            if (r2 < s.rc2) lj_pair<PREC>(a, dx, dy, dz, r2, s.potshift, rec, ptens);
+                        }
                     }
-                    const double dx = __dsub_rn(pi.x, xj);
-                    const double dy = __dsub_rn(pi.y, yj);
-                    const double dz = __dsub_rn(pi.z, zj);
-                    const double r2 = norm2_rn(dx, dy, dz);
-                    if (r2 < s.rc2) lj_pair<PREC>(a, dx, dy, dz, r2, s.potshift, rec, ptens);
+                }
+            } else {
+                for (int st = 0; row_first<TPM>(st) < cnt; st++) {
+                    const int left = row_left<TPM>(st, lane, cnt);
+                    const int4 e4 = row_entries<TPM>(L, st, lane, left);
+                    const int ev[4] = {e4.x, e4.y, e4.z, e4.w};
+                    double4 pj[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        if (left > row_off<TPM>(q)) pj[q] = ldg_pos(Pj + (ev[q] & NB_INDEX_MASK));
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        if (left <= row_off<TPM>(q)) continue;
+                        const int code = ev[q] >> NB_SHIFT_BITS;
+                        double xj = pj[q].x, yj = pj[q].y, zj = pj[q].z;
+                        if (code != NB_NOSHIFT) {  // rows of boundary cells only
+                            xj = image(xj, (code & 3) - 1, s.L[0]);
+                            yj = image(yj, ((code >> 2) & 3) - 1, s.L[1]);
+                            zj = image(zj, ((code >> 4) & 3) - 1, s.L[2]);
+                        }
+                        const double dx = __dsub_rn(pi.x, xj);
+                        const double dy = __dsub_rn(pi.y, yj);
+                        const double dz = __dsub_rn(pi.z, zj);
+                        const double r2 = norm2_rn(dx, dy, dz);
+                        if (r2 < s.rc2) lj_pair<PREC>(a, dx, dy, dz, r2, s.potshift, rec, ptens);
+                    }
                 }
             }
         }

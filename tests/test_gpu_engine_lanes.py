@@ -1,0 +1,46 @@
+"""Every number of lanes of the engine's force kernel meets each entry of a row
+once: rows of 0 to 100 entries, so every remainder of a chunk of eight."""
+import numpy as np
+import pytest
+
+from flowmol_b200 import api, lattice
+
+pytestmark = pytest.mark.gpu
+
+
+def _drop_in_gas():
+    rng = np.random.default_rng(3)
+    r, v, dom = lattice.lj_fluid([12, 12, 12], 0.9, 1.0, 85)
+    keep = (np.linalg.norm(r, axis=1) < 6.0) | (rng.random(len(r)) < 0.15)
+    return lattice.jitter(r[keep], 0.04, 86, dom), v[keep], dom
+
+
+def _row_lengths(r, v, dom):
+    s = api.MDSystem(api.make_params(len(r), dom, 2.5))
+    s.upload(r, v)
+    s.setup()
+    n = np.bincount(s.pair_list()[0] - 1, minlength=len(r))
+    s.close()
+    return n
+
+
+@pytest.mark.parametrize("tpm", [1, 2, 4, 8])
+@pytest.mark.parametrize("precision", [api.PRECISION_FP64, api.PRECISION_FP32])
+def test_lanes_agree(gpu_lib, tpm, precision):
+    """One velocity-Verlet step against the 16-lane kernel. The lanes differ in
+    the order of a sum of at most 120 FP64 terms of up to 1e3, so a differs by
+    at most 1.4e-11 and v by dt 1.4e-11 = 7e-14; an ulp of r (1.8e-15) times a
+    stiffness of 1e4 adds dt/2 1.8e-11 = 4.5e-14: below 2e-13 in all."""
+    r, v, dom = _drop_in_gas()
+    n = _row_lengths(r, v, dom)
+    assert n.min() <= 6 and n.max() > 64 and len(np.unique(n % 8)) == 8
+    out = []
+    for t in (tpm, 16):
+        e = api.Engine(8192, 40000, 8192 * 160, 2, threads_per_molecule=t, precision=precision, ticks_per_chunk=4)
+        job = e.submit(api.make_job(len(r), dom, 2.5, 1, tplot=1), r, v)
+        e.run()
+        assert e.results()[0]["status"] == 0
+        out.append(e.job_state(job, len(r)))
+        e.close()
+    for x, y in zip(*out):
+        assert np.abs(x - y).max() <= 2e-13
