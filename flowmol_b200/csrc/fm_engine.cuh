@@ -110,7 +110,7 @@ struct EngDev {
     // rebuild work list of the tick: slots, and prefix sums of their molecules
     // and cells ([rb_n + 1] each), so the rebuild kernels visit only those
     int32_t *rb_slot, *rb_mpre, *rb_cpre, *rb_upre, *rb_rpre;
-    // list_build automatic: ticks that rebuild few molecules build by molecule
+    // list_build automatic: ticks with few warps of it build by molecule (ENG_ROWS_WARPS)
     int rows_ok;
 };
 

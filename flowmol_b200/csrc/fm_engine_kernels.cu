@@ -119,6 +119,15 @@ __device__ void decide_slot(const EngDev &d, EngSlot &s)
 __device__ __forceinline__ bool slot_rebuilding(const EngSlot &s) { return slot_active(s) && s.rebuild; }
 
 constexpr int EDEC = 1024;
+// A tick builds by molecule up to this many warps of it (32 / rows_g molecules
+// each: a dense liquid's molecule is a warp, of short-range systems four share
+// one), by cell above. LJ replicas, one lane per molecule, us a tick with the
+// line at 0 / 4,096 / 16,384 / 32,768 warps: 63,756 molecules 99 / 92 / 88 /
+// 89, 150,236: 149 / 144 / 140 / 140, 193,528: 186 / 183 / 179 / 180, 316,132 and
+// more: alike; 144,720 molecules of Couette channels 91 / 91 / 92 / 94. (By
+// molecules, the single system's line: 65,536 takes 91, 145, 186 and, at
+// 316,132, 250 instead of 240.)
+constexpr int ENG_ROWS_WARPS = 16384;
 __global__ void __launch_bounds__(EDEC) k_e_decide(EngDev d)
 {
     pdl_enter();
@@ -208,7 +217,7 @@ __global__ void __launch_bounds__(EDEC) k_e_decide(EngDev d)
         d.rb_upre[carry[0]] = carry[3];
         d.rb_rpre[carry[0]] = carry[4];
         d.flags->rb_rtot = carry[4];
-        d.flags->rb_rows = d.rows_ok && carry[1] <= ROWS_MAX_MOLECULES;
+        d.flags->rb_rows = d.rows_ok && carry[4] <= ENG_ROWS_WARPS;
         d.flags->rb_n = carry[0];
         d.flags->rb_mtot = carry[1];
         d.flags->rb_ctot = carry[2];

@@ -1,5 +1,6 @@
 """Every number of lanes of the engine's force kernel meets each entry of a row
-once: rows of 0 to 100 entries, so every remainder of a chunk of eight."""
+once (rows of 0 to 100 entries, so every remainder of a chunk of eight), and
+its two list builds give the same jobs on both sides of the line between them."""
 import numpy as np
 import pytest
 
@@ -44,3 +45,32 @@ def test_lanes_agree(gpu_lib, tpm, precision):
         e.close()
     for x, y in zip(*out):
         assert np.abs(x - y).max() <= 2e-13
+
+
+# a dense liquid's molecule is a warp of the build by molecule, four molecules
+# share one at WCA range: 16,384 warps, one job more, and a mixture of both
+JOBS = {
+    "at_the_line": [([16, 16, 16], 0.8442, 2.5)],
+    "above_the_line": [([16, 17, 16], 0.8442, 2.5)],
+    "together_above": [([15, 16, 16], 0.8442, 2.5), ([8, 8, 8], 0.8, 2.5)],
+    "mixed_ranges": [([14, 15, 14], 0.8442, 2.5), ([12, 12, 13], 0.8, 2.0 ** (1.0 / 6.0)), ([10, 10, 9], 0.8, 1.45)],
+}
+
+
+@pytest.mark.parametrize("name", sorted(JOBS))
+def test_rows_by_molecule_and_by_cell_give_the_same_jobs(gpu_lib, name):
+    """Both sides of the line below which a tick builds by molecule: the same
+    rows in the same order, so the same trajectories to the last bit."""
+    out = []
+    for mode in (api.LIST_BUILD_AUTO, api.LIST_BUILD_CELLS):
+        e = api.Engine(40000, 160000, 40000 * 160, 4, threads_per_molecule=1, list_build=mode, ticks_per_chunk=8)
+        ids = []
+        for k, (nu, rho, rc) in enumerate(JOBS[name]):
+            r, v, dom = lattice.lj_fluid(nu, rho, 1.0, 91 + k)
+            ids.append((e.submit(api.make_job(len(r), dom, rc, 30, tplot=10), lattice.jitter(r, 0.04, 92, dom), v), len(r)))
+        e.run()
+        assert all(x["status"] == 0 for x in e.results())
+        out.append([e.job_state(*j) for j in ids])
+        e.close()
+    for x, y in zip(*out):
+        assert np.array_equal(x[0], y[0]) and np.array_equal(x[1], y[1])
