@@ -13,11 +13,22 @@ namespace fm {
 
 namespace {
 
+// Whether the build runs. Its grid has more blocks than fit at once, and one
+// whose row overflows raises ST_NLIST while others have yet to start: they go
+// on, so that max_nbr covers every row and one growth fits them all. (After an
+// overflow of an earlier step positions and cells stand still, and the build
+// only repeats its rows.)
+__device__ __forceinline__ bool rows_gate(const FmDev &d, int gated)
+{
+    if (*(volatile uint32_t *)&d.sc->status & (ST_FATAL & ~ST_NLIST)) return false;
+    return !gated || d.sc->rebuild;
+}
+
 template <int G>
 __global__ void __launch_bounds__(ROWS_THREADS) k_rows(FmDev d, int gated, int iter)
 {
     pdl_enter();
-    if (frozen(d) || (gated && !d.sc->rebuild)) return;
+    if (!rows_gate(d, gated)) return;
     __shared__ RowsShared<G> sh[ROWS_THREADS / 32];
     CellSys y;
     y.P = cur_pos(d, d.sc->pset);
@@ -51,7 +62,7 @@ __global__ void __launch_bounds__(ROWS_THREADS) k_rows(FmDev d, int gated, int i
 __global__ void __launch_bounds__(ROWS_THREADS) k_rows_four(FmDev d, int gated, int iter)
 {
     pdl_enter();
-    if (frozen(d) || (gated && !d.sc->rebuild)) return;
+    if (!rows_gate(d, gated)) return;
     __shared__ RowsShared<32> sh[ROWS_THREADS / 32];
     CellSys y;
     y.P = cur_pos(d, d.sc->pset);
