@@ -1009,7 +1009,7 @@ static int autotune_tpm(fm_handle *h)
         }
     }
     for (int c = 0; c < 5; c++)
-        if (tbest[c] < best) { best = tbest[c]; best_tpm = cands[c]; }
+        if (tbest[c] < fm::MORE_LANES_GAIN * best) { best = tbest[c]; best_tpm = cands[c]; }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     FM_CUDA(cudaGetLastError());

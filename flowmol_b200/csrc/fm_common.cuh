@@ -283,6 +283,15 @@ int tile_ucap_limit(int R);
 // Decodes the tiled rows into the generic int32 layout at `out` (rows of
 // d.maxn), for the pair-list and digest test hooks.
 void launch_tile_to_generic(const FmDev &d, int32_t *out, int maxn, cudaStream_t st);
+// The autotuners time forces alone, from few lanes per molecule to many, and
+// take more lanes only for a gain of 2.5%: in a step the integrator's work of a
+// molecule falls to one of its lanes, which the timing does not see. 1M
+// molecules, FP32: forces 0.2478 ms with one lane and 0.2439 with two, a step
+// 0.384 and 0.390; 255,840, FP64: 0.0667 with two and 0.0682 with four, a step
+// 0.111 and 0.1165; 389,344, FP64: 0.1075 with one and 0.1040 with two, a step
+// 0.165 and 0.164.
+constexpr float MORE_LANES_GAIN = 0.975f;
+
 // Forces: mode 0 forces only, 1 forces + move(2), 2 forces + move(2) + next
 // move(1), 3 forces + leap-frog move.
 void launch_force(const FmDev &d, int record, int mode, int tpm, cudaStream_t st);

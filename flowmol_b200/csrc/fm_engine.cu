@@ -606,7 +606,7 @@ int autotune(fm_engine *e)
         cudaEventSynchronize(b);
         float ms = 0.f;
         cudaEventElapsedTime(&ms, a, b);
-        if (ms < best) { best = ms; best_t = t; }
+        if (ms < fm::MORE_LANES_GAIN * best) { best = ms; best_t = t; }
     }
     cudaEventDestroy(a);
     cudaEventDestroy(b);
