@@ -1246,8 +1246,12 @@ void launch_tile_to_generic(const FmDev &d, int32_t *out, int maxn, cudaStream_t
 
 int force_blocks(int n, int tpm) { return nblk(n * tpm, FORCE_THREADS); }
 // Lanes per molecule: one lane's walk over all the others is what a small
-// system waits for (500 molecules: 85 us a step with one lane on two SMs).
-static int all_pairs_lanes(int n) { return n <= 8192 ? 32 : n <= 32768 ? 8 : 1; }
+// system waits for, a larger one for its blocks to fill the GPU evenly. FP64, us
+// a step with 1 / 8 / 16 / 32 lanes: 500 molecules 98 / 17 / 12 / 10, 4,000: 598
+// / 90 / 61 / 60, 6,912: 989 / 166 / 139 / 146, 8,788: 1,244 / 223 / 220 / 305, 16,384:
+// 2,314 / 649 / 875 / 884, 37,044: 5,729 / 2,456 / 3,219 / 4,036; with 1 / 8 lanes
+// 62,500: 9,806 / 6,696, 131,072: 29,232 / 27,924, 256,000: 105,890 / 104,400.
+static int all_pairs_lanes(int n) { return n <= 8192 ? 32 : 8; }
 int all_pairs_blocks(int n) { return nblk((long long)n * all_pairs_lanes(n), AP_THREADS); }
 
 void launch_force(const FmDev &d, int record, int mode, int tpm, cudaStream_t st)
