@@ -140,9 +140,25 @@ __device__ __forceinline__ double4 ldg_pos(const double4 *p)
     return r;
 }
 
+// Sorts perm[b .. b+m) by key(perm value), by one lane (insertion).
+template <typename K>
+__device__ __forceinline__ void lane_sort_cell(int32_t *perm, int b, int m, K &&key_of)
+{
+    for (int x = b + 1; x < b + m; x++) {
+        const int o = perm[x];
+        const unsigned long long key = key_of(o);
+        int y = x - 1;
+        while (y >= b && key_of(perm[y]) > key) {
+            perm[y + 1] = perm[y];
+            y--;
+        }
+        perm[y + 1] = o;
+    }
+}
+
 // Sorts perm[b .. b+m) by key(perm value), by one warp: up to 32 members by a
 // bitonic sort in registers (as many stages as they need), up to 128 by rank,
-// more by lane 0 (insertion). Keys are distinct and below 2^59.
+// more by lane 0. Keys are distinct and below 2^59.
 constexpr int SORT_RANK = 128;
 template <typename K>
 __device__ __forceinline__ void warp_sort_cell(int32_t *perm, int b, int m, int lane, K &&key_of)
@@ -186,17 +202,34 @@ __device__ __forceinline__ void warp_sort_cell(int32_t *perm, int b, int m, int 
         for (int q = 0; q < SORT_RANK / 32; q++)
             if (q * 32 + lane < m) perm[b + rank[q]] = o[q];
     } else if (lane == 0) {
-        for (int x = b + 1; x < b + m; x++) {
-            const int o = perm[x];
-            const unsigned long long key = key_of(o);
-            int y = x - 1;
-            while (y >= b && key_of(perm[y]) > key) {
-                perm[y + 1] = perm[y];
-                y--;
-            }
-            perm[y + 1] = o;
+        lane_sort_cell(perm, b, m, key_of);
+    }
+}
+
+// The same for four cells at once, each with eight lanes (lane & 7 of them,
+// with its own b and m), where m <= 8; larger ones are left as they are.
+template <typename K>
+__device__ __forceinline__ void warp_sort_four_cells(int32_t *perm, int b, int m, int lane, K &&key_of)
+{
+    const int l8 = lane & 7;
+    const bool mine = m <= 8 && l8 < m;
+    unsigned long long key = ~0ull;
+    int o = 0;
+    if (mine) {
+        o = perm[b + l8];
+        key = (m > 1 ? key_of(o) : 0ull) << 3 | (unsigned)l8;
+    }
+#pragma unroll
+    for (int k = 2; k <= 8; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, j);
+            const bool keep_min = ((l8 & j) == 0) == ((l8 & k) == 0);
+            key = keep_min ? (key < other ? key : other) : (key > other ? key : other);
         }
     }
+    o = __shfl_sync(0xffffffffu, o, (lane & 24) | (int)(key & 7u));
+    if (mine) perm[b + l8] = o;
 }
 
 template <typename T>

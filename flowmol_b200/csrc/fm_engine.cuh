@@ -62,7 +62,7 @@ struct EngFlags {
     int any_rebuild, any_list, any_ap, any_lfv, any_thermo, any_record;
     int mol_hwm, cell_hwm;
     // this tick's rebuilding jobs (slot order): count, their molecules, their
-    // cells, their list-build units (cells or 2x2x2 blocks)
+    // cell-sort units (cells, or four cells), their list-build units (cells or 2x2x2 blocks)
     int rb_n, rb_mtot, rb_ctot, rb_utot;
     // list build by molecule this tick (fm_rows.cuh), and its units (warps)
     int rb_rows, rb_rtot;
@@ -108,7 +108,7 @@ struct EngDev {
     double *red_part;
     int32_t *red_count;
     // rebuild work list of the tick: slots, and prefix sums of their molecules
-    // and cells ([rb_n + 1] each), so the rebuild kernels visit only those
+    // and units ([rb_n + 1] each), so the rebuild kernels visit only those
     int32_t *rb_slot, *rb_mpre, *rb_cpre, *rb_upre, *rb_rpre;
     // list_build automatic: ticks with few warps of it build by molecule (ENG_ROWS_WARPS)
     int rows_ok;

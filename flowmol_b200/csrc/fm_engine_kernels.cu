@@ -118,6 +118,9 @@ __device__ void decide_slot(const EngDev &d, EngSlot &s)
 
 __device__ __forceinline__ bool slot_rebuilding(const EngSlot &s) { return slot_active(s) && s.rebuild; }
 
+// Cells of a sparse job (two or three molecules each) are sorted four a warp.
+__device__ __forceinline__ bool sort_by_four(const EngSlot &s) { return s.rows_g == 8; }
+
 constexpr int EDEC = 1024;
 // A tick builds by molecule up to this many warps of it (32 / rows_g molecules
 // each: a dense liquid's molecule is a warp, of short-range systems four share
@@ -165,7 +168,7 @@ __global__ void __launch_bounds__(EDEC) k_e_decide(EngDev d)
             if (slot_rebuilding(s)) {
                 x[0] = 1;
                 x[1] = s.nmol;
-                x[2] = s.mode == MODE_LIST ? s.ncell : 0;
+                x[2] = s.mode != MODE_LIST ? 0 : sort_by_four(s) ? (s.ncell + 3) / 4 : s.ncell;
                 x[3] = s.mode != MODE_LIST ? 0
                        : s.build_blocks ? ((s.ne[0] + 1) / 2) * ((s.ne[1] + 1) / 2) * ((s.ne[2] + 1) / 2)
                                         : s.ncell;
@@ -343,28 +346,47 @@ __global__ void k_e_scatter(EngDev d)
     }
 }
 
-// Cell by cell, one warp each: by octant, then by the order the molecules had
-// (the single-system cell sort, fm_kernels.cu, goes by identity instead).
-__global__ void k_e_sort(EngDev d)
+// Cell by cell: by octant, then by the order the molecules had (the
+// single-system cell sort, fm_kernels.cu, goes by identity instead). A warp
+// takes a cell, or four of a sparse job: with a warp for each of those a tick of
+// 16 Couette channels (144,720 molecules, 2.3 a cell) took 92 us instead of 88,
+// of 48 (395,020) 164 instead of 156. 48 registers: at 54 the dense jobs' sort
+// lost a block an SM, 243 -> 249 us a tick at 316,132 LJ molecules.
+__global__ void __launch_bounds__(256, 5) k_e_sort(EngDev d)
 {
     pdl_enter();
     if (!d.flags->any_rebuild) return;
     const int tot = d.flags->rb_ctot, lane = threadIdx.x & 31;
     int r = 0;
     for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < tot; g += (gridDim.x * blockDim.x) >> 5) {
-        const int lc = rb_entry(d.rb_cpre, g, r);
+        const int unit = rb_entry(d.rb_cpre, g, r);
         EngSlot &s = d.slots[d.rb_slot[r]];
-        const int c = s.cell_off + lc;
-        const int b = d.cell_start[s.cstart_off + lc], e = d.cell_start[s.cstart_off + lc + 1];
-        if (lane == 0) d.cell_count[c] = 0;
-        if (b == e) continue;
         const double4 *P = eng_pos(d, s.pset);
+        const bool four = sort_by_four(s);
+        const int lc = four ? 4 * unit + (lane >> 3) : unit;
+        const bool in = lc < s.ncell;
+        const int c = s.cell_off + lc;
+        const int b = in ? d.cell_start[s.cstart_off + lc] : 0, m = in ? d.cell_start[s.cstart_off + lc + 1] - b : 0;
         const int cx = lc % s.ne[0], cy = (lc / s.ne[0]) % s.ne[1], cz = lc / (s.ne[0] * s.ne[1]);
-        warp_sort_cell(d.perm, b, e - b, lane, [&](int o) {
+        auto key_of = [&](int o) {
             return (unsigned long long)sub_cell(P[o], cx, cy, cz, s.hd, s.cs) << 32 | (unsigned)o;
-        });
-        for (int k = b + lane; k < e; k += 32) d.cell_of[k] = c;  // by new index from here on
-        if (lane == 0 && (is_halo(cx, s.ne[0]) || is_halo(cy, s.ne[1]) || is_halo(cz, s.ne[2]))) s.strays = 1;
+        };
+        if (in && (lane & (four ? 7 : 31)) == 0) {
+            d.cell_count[c] = 0;
+            if (m > 0 && (is_halo(cx, s.ne[0]) || is_halo(cy, s.ne[1]) || is_halo(cz, s.ne[2]))) s.strays = 1;
+        }
+        if (!four) {
+            warp_sort_cell(d.perm, b, m, lane, key_of);
+            for (int k = lane; k < m; k += 32) d.cell_of[b + k] = c;  // by new index from here on
+            continue;
+        }
+        warp_sort_four_cells(d.perm, b, m, lane, key_of);
+        if (m <= 8 && (lane & 7) < m) d.cell_of[b + (lane & 7)] = c;
+        // a cell of more than eight: by one of its lanes
+        if (m > 8 && (lane & 7) == 0) {
+            lane_sort_cell(d.perm, b, m, key_of);
+            for (int k = 0; k < m; k++) d.cell_of[b + k] = c;
+        }
     }
 }
 

@@ -396,27 +396,8 @@ __global__ void __launch_bounds__(32 * SORT_WARPS) k_sort_cells_sparse(FmDev d, 
         const int c = c0 + (lane >> 3);
         const bool in = c < d.ncell;
         const int b = in ? d.cell_start[c] : 0, m = in ? d.cell_start[c + 1] - b : 0;
-        const bool mine = m <= 8 && l8 < m;
-        unsigned long long key = ~0ull;
-        int o = 0;
-        if (mine) {
-            o = d.perm[b + l8];
-            key = (m > 1 ? sort_key(d, P, o, c) : 0ull) << 3 | (unsigned)l8;
-        }
-#pragma unroll
-        for (int k = 2; k <= 8; k <<= 1) {
-#pragma unroll
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, j);
-                const bool keep_min = ((l8 & j) == 0) == ((l8 & k) == 0);
-                key = keep_min ? (key < other ? key : other) : (key > other ? key : other);
-            }
-        }
-        o = __shfl_sync(0xffffffffu, o, (lane & 24) | (int)(key & 7u));
-        if (mine) {
-            d.perm[b + l8] = o;
-            d.cell_of[b + l8] = c;  // by new slot from here on
-        }
+        warp_sort_four_cells(d.perm, b, m, lane, [&](int o) { return sort_key(d, P, o, c); });
+        if (m <= 8 && l8 < m) d.cell_of[b + l8] = c;  // by new slot from here on
         if (in && l8 == 0) sorted_cell(d, c, m);
         for (unsigned large = __ballot_sync(0xffffffffu, l8 == 0 && m > 8); large != 0u; large &= large - 1u) {
             const int from = __ffs(large) - 1;
