@@ -33,6 +33,8 @@ __device__ __forceinline__ unsigned long long bead_key(int chain, int sub)
 {
     return (unsigned long long)(unsigned)chain << 32 | (unsigned)sub;
 }
+// The finaliser of splitmix64 (Steele, Lea and Flood, OOPSLA 2014) with other
+// shifts and without its last one: the upper half of the product is taken.
 __device__ __forceinline__ unsigned bead_hash(unsigned long long x)
 {
     x ^= x >> 29; x *= 0xbf58476d1ce4e5b9ull;

@@ -1,5 +1,5 @@
 // fm_build.cuh -- the neighbour-list build of one cell, shared by the
-// single-system kernel (fm_kernels.cu) and the slot engine
+// single-system kernel (fm_build.cu) and the slot engine
 // (fm_engine_kernels.cu).
 //
 // Pair set of assign_to_neighbourlist_halfint_opt (linklist.f90:660-804,

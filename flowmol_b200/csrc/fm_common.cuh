@@ -264,8 +264,10 @@ void launch_scan_cells(const FmDev &d, int gated, cudaStream_t st);
 void launch_scatter(const FmDev &d, int gated, cudaStream_t st);
 void launch_reorder(const FmDev &d, int gated, double4 *tpos, int32_t *tuidx, cudaStream_t st);
 void launch_build_nlist(const FmDev &d, int gated, int iter, cudaStream_t st);
-// The same rows by molecule (fm_rows.cu), for up to ROWS_MAX_MOLECULES: 32,000
-// molecules 64 us against ~130 by warp, 108,000 170 against 160.
+// The same rows by molecule (fm_rows.cu), for up to ROWS_MAX_MOLECULES. The
+// build kernel alone, LJ liquid: 2,048 molecules 14 us against 89 by warp, 16,384
+// 46 against 88, 32,000 66 against 106, 65,000 110 against 119, 108,000 170
+// against 155.
 constexpr int ROWS_MAX_MOLECULES = 65536;
 void launch_rows(const FmDev &d, int gated, int iter, cudaStream_t st);
 // Bonds (potential_flag 1): the bead table at upload, the bonds after each build.

@@ -14,17 +14,18 @@
 // per lane and left in shared memory), G candidates a step: each lane loads one
 // position and makes the exact test, the step's hits are one ballot, and a
 // hit's place in the row is the count so far plus its rank in the ballot, so
-// rows are in visiting order without any buffer. G is the power of two nearest
-// the length of a range.
+// rows are in visiting order without any buffer. G is 32 for ranges of more than
+// 20 candidates, 16 above 10, else 8 (rows_lanes).
 //
 // It is for systems that do not fill the GPU: the chain of steps of one
 // molecule is short, where the build by warp (fm_build.cuh: a cell, or 2x2x2 of
-// them, per warp) waits for the serial work of one warp, ~100 us however small
-// the system is: a rebuild of 2,048 LJ molecules costs 34 us instead of 132,
-// one of 32,000 90 instead of 152 (by fours, below). Bound by issue at larger
-// sizes (some 80 instructions a step, 8 of them FP64): at 108,000 molecules 170
-// us by fours and 264 by molecule against 160 by warp, whose staging in shared
-// memory tests four owners per candidate loaded.
+// them, per warp) waits for the serial work of one warp, ~90 us however small
+// the system is: a whole rebuild (cells, sort, reorder, rows) of 2,048 LJ
+// molecules takes 34 us instead of 132, one of 32,000 90 instead of 152 (by
+// fours, below). Bound by issue at larger sizes (some 80 instructions a step, 8
+// of them FP64): the kernel alone takes 170 us by fours and 264 by molecule at
+// 108,000 molecules against 155 by warp, whose staging in shared memory tests
+// four owners per candidate loaded.
 #pragma once
 #include "fm_build.cuh"
 
@@ -219,7 +220,7 @@ __device__ __forceinline__ int rows_four(const CellSys &y, int i0, int own, int 
 // halo cells have molecules (strays, or a subdomain's copies, which get no
 // rows), the first of a cell's warps looks after an equal share of them.
 constexpr int ROWS_SPLIT = 5;
-constexpr int ROWS_FOUR_MOLECULES = 16384;  // a warp's chain is longer: 2,048 molecules 50 us a rebuild against 34
+constexpr int ROWS_FOUR_MOLECULES = 16384;  // a warp's chain is longer: a whole rebuild of 2,048 molecules 50 us against 34
 __host__ __device__ inline int rows_four_units(const int (&ne)[3])
 {
     return (ne[0] - 2) * (ne[1] - 2) * (ne[2] - 2) * ROWS_SPLIT;
